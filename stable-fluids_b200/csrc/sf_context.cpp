@@ -324,7 +324,9 @@ struct Stages {
     // 3. implicit viscosity, x0 = advected velocity (:621-641).
     void diffuse_velocity() {
         if (!(alpha_v() > 0.0f)) return;
-        for (int comp = 0; comp < 3; ++comp) ok(launch_stencil(stencil(KIND_VEL_X + comp, INIT_FROM_B, c.config.diffuse_iterations, alpha_v(), c.vel[comp], c.temp[comp]), c.stream), 0);
+        StencilArgs solves[3];
+        for (int comp = 0; comp < 3; ++comp) solves[comp] = stencil(KIND_VEL_X + comp, INIT_FROM_B, c.config.diffuse_iterations, alpha_v(), c.vel[comp], c.temp[comp]);
+        ok(launch_stencils(solves, 3, c.stream), 0);
     }
 
     // 4. divergence (:643).

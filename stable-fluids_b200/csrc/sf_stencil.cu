@@ -1408,7 +1408,16 @@ bool launch_residual_sums_vec(const float* p, const float* div, Dims d, float h2
     return true;
 }
 
+cudaError_t launch_stencils(const StencilArgs* a, int n, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    if (launch_resident(a, n, s, &e)) return e;
+    for (int k = 0; k < n && e == cudaSuccess; ++k) e = launch_stencil(a[k], s);
+    return e;
+}
+
 cudaError_t launch_stencil(const StencilArgs& a, cudaStream_t s) {
+    cudaError_t resident = cudaSuccess;
+    if (launch_resident(&a, 1, s, &resident)) return resident;
     // per_pass: 0 (default) = one launch per Jacobi sweep, red-black solves
     // in the colour-split layout where the rows allow (one launch per
     // colour); 1 = one launch per sweep or per colour on the interleaved

@@ -18,9 +18,8 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
-#include <cstdlib>
-#include <cstring>
 #include <memory>
 #include <mutex>
 #include <new>
@@ -32,7 +31,7 @@
 #include "sf_unet.h"
 #include "sf_unet_kernels.cuh"
 #include "sf_unet_tc.cuh"
-#include "sf_unet_wgrad_tc.cuh"
+#include "sf_unet_wgrad.cuh"
 #include "stable-fluids-b200.h"
 
 namespace sfb::net {
@@ -123,6 +122,18 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
+// 4-D map over a channels-last tensor of C channels, boxes of 8 channels x
+// bx x by x bz voxels.
+bool voxel_map(CUtensorMap* m, const __nv_bfloat16* base, int C, Dims d, int bx, int by, int bz) {
+    auto encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
+    const cuuint64_t gd[4] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(d.nx), static_cast<cuuint64_t>(d.ny), static_cast<cuuint64_t>(d.nz)};
+    const cuuint64_t gs[3] = {static_cast<cuuint64_t>(C) * 2, static_cast<cuuint64_t>(d.nx) * C * 2, static_cast<cuuint64_t>(d.ny) * d.nx * C * 2};
+    const cuuint32_t box[4] = {8u, static_cast<cuuint32_t>(bx), static_cast<cuuint32_t>(by), static_cast<cuuint32_t>(bz)};
+    const cuuint32_t es[4] = {1u, 1u, 1u, 1u};
+    return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(base), gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int sm_count() {
     static const int n = [] {
         int dev = 0, v = 148;
@@ -130,6 +141,18 @@ int sm_count() {
         return v;
     }();
     return n;
+}
+
+// 2-D map over the same tensor as (channel, voxel), boxes of 16 channels x
+// `rows` voxels, 32-byte swizzle.
+bool rows_map(CUtensorMap* m, const __nv_bfloat16* base, int C, long long voxels, int rows) {
+    auto encode = tensor_map_encoder();
+    if (encode == nullptr) return false;
+    const cuuint64_t gd[2] = {static_cast<cuuint64_t>(C), static_cast<cuuint64_t>(voxels)};
+    const cuuint64_t gs[1] = {static_cast<cuuint64_t>(C) * 2};
+    const cuuint32_t box[2] = {16u, static_cast<cuuint32_t>(rows)};
+    const cuuint32_t es[2] = {1u, 1u};
+    return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(base), gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // 3x3x3 convolution on the tensor cores (tc::k_conv3d_tc): tensor maps for
@@ -143,12 +166,7 @@ cudaError_t conv(const __nv_bfloat16* in, const __nv_bfloat16* w, const float* b
     auto encode = tensor_map_encoder();
     if (encode == nullptr) return cudaErrorNotSupported;
     CUtensorMap map_in{}, map_w{};
-    const cuuint64_t gd[4] = {static_cast<cuuint64_t>(CIN), static_cast<cuuint64_t>(d.nx), static_cast<cuuint64_t>(d.ny), static_cast<cuuint64_t>(d.nz)};
-    const cuuint64_t gs[3] = {static_cast<cuuint64_t>(CIN) * 2, static_cast<cuuint64_t>(d.nx) * CIN * 2, static_cast<cuuint64_t>(d.ny) * d.nx * CIN * 2};
-    const cuuint32_t box[4] = {8u, static_cast<cuuint32_t>(tc::P), static_cast<cuuint32_t>(C::TY + 2), 1u};
-    const cuuint32_t es[4] = {1u, 1u, 1u, 1u};
-    if (encode(&map_in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(in), gd, gs, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
+    if (!voxel_map(&map_in, in, CIN, d, tc::P, C::TY + 2, 1)) return cudaErrorInvalidValue;
     const cuuint64_t tap = static_cast<cuuint64_t>(COUT) * CIN * 2;  // bytes per tap
     const cuuint64_t wd[5] = {static_cast<cuuint64_t>(CIN), static_cast<cuuint64_t>(COUT), 3u, 3u, 3u};
     const cuuint64_t ws[4] = {static_cast<cuuint64_t>(CIN) * 2, tap, 3 * tap, 9 * tap};
@@ -180,44 +198,55 @@ cudaError_t conv_any(int cin, int cout, int epi, const __nv_bfloat16* in, const 
     return cudaErrorInvalidValue;
 }
 
-// The weight gradient on the tcgen05 tensor cores (sf_unet_wgrad_tc.cuh);
-// STABLE_FLUIDS_B200_WGRAD=mma selects the mma.sync GEMM per tap instead.
-bool wgrad_on_mma_sync() {
-    static const bool v = [] {
-        const char* e = std::getenv("STABLE_FLUIDS_B200_WGRAD");
-        return e != nullptr && std::strcmp(e, "mma") == 0;
-    }();
-    return v;
-}
-
+// The weight gradient of a layer (sf_unet_wgrad.cuh): CTAs of 16 input
+// channels, one CTA per SM over the channel groups.
 template <int CIN, int COUT>
 cudaError_t wgrad(const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw, float* db, Dims d, cudaStream_t s, unsigned* error) {
-    if (wgrad_on_mma_sync() || static_cast<long long>(d.nx) * d.ny * d.nz >= (1ll << 31)) {  // the tensor-core form indexes voxels in 32 bits
-        const int zper = d.nz >= 64 ? 4 : (d.nz >= 16 ? 2 : 1);
-        const dim3 grid(27, static_cast<unsigned>((d.nz + zper - 1) / zper));
-        k_conv3d_wgrad<CIN, COUT><<<grid, 128, 0, s>>>(in, dout, dw, db, d, zper);
-        return cudaGetLastError();
-    }
-    using C = tc::WgCfg<CIN, COUT>;
-    const auto kern = tc::k_conv3d_wgrad_tc<CIN, COUT>;
+    using C = wg::Cfg<COUT>;
+    CUtensorMap map_in{}, map_out{};
+    if (!voxel_map(&map_in, in, CIN, d, wg::TX + 2, wg::TY + 2, C::TZ + 2) || !voxel_map(&map_out, dout, COUT, d, wg::TX, wg::TY, C::TZ)) return cudaErrorInvalidValue;
+    const auto kern = wg::k_conv3d_wgrad<COUT>;
     static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES);
     if (attr != cudaSuccess) return attr;
-    static const int per_sm = [&] {
-        int k = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, tc::kWgThreads, C::BYTES) != cudaSuccess || k < 1) k = 1;
-        return k;
-    }();
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const long long nvox = static_cast<long long>(d.nx) * d.ny * d.nz;
-    const long long nchunks = (nvox + tc::kWgK - 1) / tc::kWgK;
-    long long per_tap = static_cast<long long>(sms) * per_sm / 27;  // one wave of CTAs over the 27 taps
-    if (per_tap < 1) per_tap = 1;
-    const long long chunks = (nchunks + per_tap - 1) / per_tap;
-    const dim3 grid(27, static_cast<unsigned>((nchunks + chunks - 1) / chunks));
-    kern<<<grid, tc::kWgThreads, C::BYTES, s>>>(in, dout, dw, db, d, static_cast<int>(chunks), error);
+    constexpr int groups = CIN / 16;
+    const int tx = (d.nx + wg::TX - 1) / wg::TX, ty = (d.ny + wg::TY - 1) / wg::TY, tz = (d.nz + C::TZ - 1) / C::TZ;
+    const wg::Args a{dw, db, CIN, tx, ty, tx * ty * tz, error};
+    const int per_group = std::max(1, std::min(a.tiles, sm_count() / groups));
+    kern<<<dim3(static_cast<unsigned>(per_group), groups), wg::kThreads, C::BYTES, s>>>(map_in, map_out, a);
     return cudaGetLastError();
 }
+
+// The weight gradients of the layers of 16 output channels, all in one launch
+// (their chains are long and narrow: 45 CTAs a layer and 16 input channels).
+struct ChainLaunch {
+    wg::ChainArgs a{};
+    int groups = 0;
+    bool ok = true;
+    void add(const __nv_bfloat16* in, int cin, const __nv_bfloat16* dout, float* dw, float* db, long long voxels) {
+        for (int c0 = 0; c0 < cin; c0 += 16) {
+            wg::ChainGroup& g = a.group[groups++];
+            ok = ok && rows_map(&g.in, in, cin, voxels, wg::ChainCfg::BOX) && rows_map(&g.rest, in, cin, voxels, 8) && rows_map(&g.out, dout, 16, voxels, wg::ChainCfg::BOX);
+            g.dw = dw;
+            g.db = c0 == 0 ? db : nullptr;
+            g.cin = cin;
+            g.c0 = c0;
+        }
+    }
+    cudaError_t launch(Dims d, cudaStream_t s, unsigned* error) {
+        if (!ok) return cudaErrorInvalidValue;
+        static const cudaError_t attr = cudaFuncSetAttribute(wg::k_conv3d_wgrad_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, wg::ChainCfg::BYTES);
+        if (attr != cudaSuccess) return attr;
+        const int voxels = d.nx * d.ny * d.nz;
+        const int units = (voxels + wg::kSegmentUnit - 1) / wg::kSegmentUnit;
+        const int segments = std::max(1, sm_count() / 27), per = (units + segments - 1) / segments;
+        a.d = d;
+        a.nvox = voxels;
+        a.segment = per * wg::kSegmentUnit;
+        a.error = error;
+        wg::k_conv3d_wgrad_chain<<<dim3(static_cast<unsigned>((units + per - 1) / per), 9, static_cast<unsigned>(groups)), wg::kChainThreads, wg::ChainCfg::BYTES, s>>>(a);
+        return cudaGetLastError();
+    }
+};
 
 cudaError_t wgrad_any(int cin, int cout, const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw, float* db, Dims d, cudaStream_t s, unsigned* error) {
 #define SFB_WG(CI, CO) \
@@ -410,15 +439,20 @@ cudaError_t backward(Net* n, cudaStream_t s) {
     Buffers& B = *n->buf;
     cudaError_t e;
     SFB_TRY(cudaMemsetAsync(n->g, 0, n->nparams * sizeof(float), s));
+    const bool chained = B.n0 < (1ull << 31) - 4096;  // the chain kernel counts voxels in 32 bits
+    ChainLaunch chain;
     // out layer (linear)
-    SFB_TRY(wgrad_any(16, 16, B.d0b, B.g16, GW(n, OUT), GB(n, OUT), B.d0, s, n->error));
+    if (chained) chain.add(B.d0b, 16, B.g16, GW(n, OUT), GB(n, OUT), static_cast<long long>(B.n0));
+    else SFB_TRY(wgrad_any(16, 16, B.d0b, B.g16, GW(n, OUT), GB(n, OUT), B.d0, s, n->error));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.g16, WT(n, OUT), nullptr, B.gd0b, 16, 0, B.d0, s, n->error));
     // d0b, d0a (input of d0a: cat0 = [up(d1b) | e0b])
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.gd0b, B.d0b, B.n0 * 16);
-    SFB_TRY(wgrad_any(16, 16, B.d0a, B.gd0b, GW(n, D0B), GB(n, D0B), B.d0, s, n->error));
+    if (chained) chain.add(B.d0a, 16, B.gd0b, GW(n, D0B), GB(n, D0B), static_cast<long long>(B.n0));
+    else SFB_TRY(wgrad_any(16, 16, B.d0a, B.gd0b, GW(n, D0B), GB(n, D0B), B.d0, s, n->error));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.gd0b, WT(n, D0B), nullptr, B.gd0a, 16, 0, B.d0, s, n->error));
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.gd0a, B.d0a, B.n0 * 16);
-    SFB_TRY(wgrad_any(48, 16, B.cat0, B.gd0a, GW(n, D0A), GB(n, D0A), B.d0, s, n->error));
+    if (chained) chain.add(B.cat0, 48, B.gd0a, GW(n, D0A), GB(n, D0A), static_cast<long long>(B.n0));
+    else SFB_TRY(wgrad_any(48, 16, B.cat0, B.gd0a, GW(n, D0A), GB(n, D0A), B.d0, s, n->error));
     SFB_TRY(conv_any(16, 48, tc::LINEAR_BF16, B.gd0a, WT(n, D0A), nullptr, B.gcat0, 48, 0, B.d0, s, n->error));
     k_upsample2_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat0, 48, 0, 32, B.d1, B.gd1b);
     // d1b, d1a (input of d1a: cat1 = [up(bb) | e1b])
@@ -449,10 +483,13 @@ cudaError_t backward(Net* n, cudaStream_t s) {
     k_copy_channels<<<blocks_for(B.n0 * 2), 256, 0, s>>>(B.gcat0, 48, 32, B.ge0b, 16, 0, 16, B.n0, 0);
     k_pool2_backward<<<row_grid(B.d0.nx, 2, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.gp0, 16, B.d1, B.ge0b, 16, 0, 1);
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.ge0b, B.e0b, B.n0 * 16);
-    SFB_TRY(wgrad_any(16, 16, B.e0a, B.ge0b, GW(n, E0B), GB(n, E0B), B.d0, s, n->error));
+    if (chained) chain.add(B.e0a, 16, B.ge0b, GW(n, E0B), GB(n, E0B), static_cast<long long>(B.n0));
+    else SFB_TRY(wgrad_any(16, 16, B.e0a, B.ge0b, GW(n, E0B), GB(n, E0B), B.d0, s, n->error));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.ge0b, WT(n, E0B), nullptr, B.ge0a, 16, 0, B.d0, s, n->error));
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.ge0a, B.e0a, B.n0 * 16);
-    SFB_TRY(wgrad_any(16, 16, B.in, B.ge0a, GW(n, E0A), GB(n, E0A), B.d0, s, n->error));
+    if (chained) chain.add(B.in, 16, B.ge0a, GW(n, E0A), GB(n, E0A), static_cast<long long>(B.n0));
+    else SFB_TRY(wgrad_any(16, 16, B.in, B.ge0a, GW(n, E0A), GB(n, E0A), B.d0, s, n->error));
+    if (chained) SFB_TRY(chain.launch(B.d0, s, n->error));
     return cudaGetLastError();
 }
 

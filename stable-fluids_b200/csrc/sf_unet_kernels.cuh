@@ -1,14 +1,12 @@
 // sf_unet_kernels.cuh -- kernels of the warm-start network besides the
-// tcgen05 convolution (sf_unet_tc.cuh): the weight gradient of a 3x3x3
-// convolution (mma.sync BF16 x BF16 -> FP32), 2x average pooling, 2x nearest
-// upsampling, and the element-wise pieces of training.
+// convolution (sf_unet_tc.cuh) and its weight gradient (sf_unet_wgrad.cuh): 2x
+// average pooling, 2x nearest upsampling, and the element-wise pieces of
+// training.
 //
 // Activations are channels-last BF16: element (voxel v, channel c) at
 // v * C + c, v = x + nx (y + ny z), C a multiple of 16 (padded with zeros).
 // Weights are BF16 [tap][cout][cin] with tap = (dz+1)*9 + (dy+1)*3 + (dx+1),
 // plus an FP32 master copy for the optimizer. Zero padding at the grid edge.
-//
-// Weight-gradient GEMM instruction: mma.sync m16n8k16 BF16 x BF16 -> FP32.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -19,85 +17,6 @@
 #include "sf_types.h"
 
 namespace sfb::net {
-
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
-
-// Weight gradient: dw[tap][co][ci] += sum_v dout[v][co] in[v + off(tap)][ci],
-// dbias[co] += sum_v dout[v][co]. GEMM per tap with M = COUT, N = CIN,
-// K = voxels; the operand tiles are stored channel-major in shared memory so
-// that K pairs are contiguous. Grid: (27, chunks); each CTA covers a z range
-// of the grid for its tap and adds its FP32 partial sums atomically.
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv3d_wgrad(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dout, float* __restrict__ dw, float* __restrict__ dbias, Dims d, int z_per_cta) {
-    static_assert(CIN % 8 == 0 && COUT % 16 == 0, "channel padding");
-    constexpr int MT = COUT / 16, NTL = CIN / 8;  // m tiles, n tiles
-    constexpr int TILES = MT * NTL;
-    constexpr int PER_WARP = (TILES + 3) / 4;
-    constexpr int V = 64;  // voxels per chunk: one row of 64 x (K = 4 x 16)
-    __shared__ __align__(16) __nv_bfloat16 sa[COUT][V + 8];
-    __shared__ __align__(16) __nv_bfloat16 sb[CIN][V + 8];
-    const int tap = static_cast<int>(blockIdx.x);
-    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-    const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
-    float acc[PER_WARP][4];
-#pragma unroll
-    for (int i = 0; i < PER_WARP; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0f;
-    float bsum = 0.0f;
-    const int zb = static_cast<int>(blockIdx.y) * z_per_cta, ze = min(zb + z_per_cta, d.nz);
-    for (int z = zb; z < ze; ++z)
-        for (int y = 0; y < d.ny; ++y)
-            for (int xc = 0; xc < d.nx; xc += V) {
-                __syncthreads();
-                for (int i = tid; i < V * COUT; i += 128) {
-                    const int c = i % COUT, vx = i / COUT, gx = xc + vx;
-                    sa[c][vx] = gx < d.nx ? dout[(static_cast<size_t>(gx) + static_cast<size_t>(d.nx) * (y + static_cast<size_t>(d.ny) * z)) * COUT + c] : __float2bfloat16(0.0f);
-                }
-                const int sy = y + dy, sz = z + dz;
-                for (int i = tid; i < V * CIN; i += 128) {
-                    const int c = i % CIN, vx = i / CIN, sx = xc + vx + dx;
-                    const bool inb = xc + vx < d.nx && static_cast<unsigned>(sx) < static_cast<unsigned>(d.nx) && static_cast<unsigned>(sy) < static_cast<unsigned>(d.ny) && static_cast<unsigned>(sz) < static_cast<unsigned>(d.nz);
-                    sb[c][vx] = inb ? in[(static_cast<size_t>(sx) + static_cast<size_t>(d.nx) * (sy + static_cast<size_t>(d.ny) * sz)) * CIN + c] : __float2bfloat16(0.0f);
-                }
-                __syncthreads();
-                if (tap == 13 && tid < COUT)
-                    for (int vx = 0; vx < V; ++vx) bsum += __bfloat162float(sa[tid][vx]);
-#pragma unroll
-                for (int kc = 0; kc < V / 16; ++kc) {
-#pragma unroll
-                    for (int i = 0; i < PER_WARP; ++i) {
-                        const int tile_id = warp * PER_WARP + i;
-                        if (tile_id >= TILES) continue;
-                        const int mt = tile_id / NTL, nt = tile_id % NTL;
-                        const int k0 = kc * 16 + 2 * t;
-                        const uint32_t a0 = ld32(&sa[mt * 16 + g][k0]), a1 = ld32(&sa[mt * 16 + g + 8][k0]);
-                        const uint32_t a2 = ld32(&sa[mt * 16 + g][k0 + 8]), a3 = ld32(&sa[mt * 16 + g + 8][k0 + 8]);
-                        const uint32_t b0 = ld32(&sb[nt * 8 + g][k0]), b1 = ld32(&sb[nt * 8 + g][k0 + 8]);
-                        mma_bf16(acc[i], a0, a1, a2, a3, b0, b1);
-                    }
-                }
-            }
-#pragma unroll
-    for (int i = 0; i < PER_WARP; ++i) {
-        const int tile_id = warp * PER_WARP + i;
-        if (tile_id >= TILES) continue;
-        const int mt = tile_id / NTL, nt = tile_id % NTL;
-        float* base = dw + static_cast<size_t>(tap) * COUT * CIN;
-        const int co = mt * 16 + g, ci = nt * 8 + 2 * t;
-        atomicAdd(base + co * CIN + ci, acc[i][0]);
-        atomicAdd(base + co * CIN + ci + 1, acc[i][1]);
-        atomicAdd(base + (co + 8) * CIN + ci, acc[i][2]);
-        atomicAdd(base + (co + 8) * CIN + ci + 1, acc[i][3]);
-    }
-    if (tap == 13 && tid < COUT && dbias) atomicAdd(dbias + tid, bsum);
-}
-
 
 // ------------------------------------------------------ element-wise pieces --
 

@@ -43,7 +43,14 @@ __device__ __forceinline__ bool easy(float4 n, const Divisor& v) {
     return small >= v.lo && big <= 0x1p126f;
 }
 
-// RN(n / d) for a pair that easy() allows.
+// RN(n / d) for an n, or a pair, that easy() allows.
+template <bool SIX>
+__device__ __forceinline__ float quotient(float n, const Divisor& v) {
+    const float q0 = __fmul_rn(n, v.y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-q0, v.d, n), v.y, q0);
+    if constexpr (SIX) return q1;
+    return __fmaf_rn(__fmaf_rn(-q1, v.d, n), v.y, q1);
+}
 template <bool SIX>
 __device__ __forceinline__ F2 quotient(F2 n, const Divisor& v) {
     const F2 y = f2(v.y, v.y), d = f2(-v.d, -v.d);
@@ -53,15 +60,20 @@ __device__ __forceinline__ F2 quotient(F2 n, const Divisor& v) {
     return fma2(fma2(q1, d, n), y, q1);
 }
 
-// RN(n / d) for four numerators; SIX: d is 6.
+// RN(n / d) for four numerators, any of them.
+__device__ __forceinline__ float4 hard(float4 n, const Divisor& v) {
+    if (n.x == 0.0f && n.y == 0.0f && n.z == 0.0f && n.w == 0.0f) return n;  // the far field
+    return make_float4(tb::divide(n.x, v.d, v.y64), tb::divide(n.y, v.d, v.y64), tb::divide(n.z, v.d, v.y64), tb::divide(n.w, v.d, v.y64));
+}
+
+// The same, the FP32 form where it serves; SIX: d is 6.
 template <bool SIX>
 __device__ __forceinline__ float4 four(float4 n, const Divisor& v) {
     if (easy(n, v)) [[likely]] {
         const F4 p = f4(n);
         return unpack(F4{quotient<SIX>(p.lo, v), quotient<SIX>(p.hi, v)});
     }
-    if (n.x == 0.0f && n.y == 0.0f && n.z == 0.0f && n.w == 0.0f) return n;  // the far field
-    return make_float4(tb::divide(n.x, v.d, v.y64), tb::divide(n.y, v.d, v.y64), tb::divide(n.z, v.d, v.y64), tb::divide(n.w, v.d, v.y64));
+    return hard(n, v);
 }
 
 }  // namespace sfb::divide

@@ -17,6 +17,7 @@
 
 #include "sf_batch.cuh"
 #include "sf_device.cuh"
+#include "sf_divide.cuh"
 #include "sf_launch.h"
 #include "sf_stencil_tb.cuh"
 #include "sf_stencil_wave.cuh"
@@ -537,84 +538,109 @@ __global__ void __launch_bounds__(256) k_rb_layout(T* __restrict__ field, T* __r
 // come from L1. No thread reads another's cells of u, so the update is in
 // place. Threads are numbered along the half plane (blockIdx.x, 128 groups
 // of four a CTA; blockIdx.z the z chunk), so short rows still fill every
-// lane of a warp.
-template <int KIND, typename T>
-__device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, const T* __restrict__ v, const T* __restrict__ w, float coef, int colour, int z_chunk, const Dims& d, const GhostRule& g, bool down = false) {
+// lane of a warp. DOWN marches the chunk from its top plane: consecutive
+// launches alternate, so that each starts on the planes the one before wrote
+// last (see jacobi_vec4_block).
+//
+// Every warp waits for its plane's loads and then issues its instructions
+// beside eight other warps of its scheduler, so the instructions a plane takes
+// bound it as much as the loads: 185 for four cells when the addresses were 64
+// bits, the quotient FP64 (tb::divide) and the direction a kernel argument.
+// With 32-bit byte offsets, the FP32 quotient and its test after the store
+// (divide::easy; a branch before the store would hold it back), a colour at
+// 256^3 takes 18.8 us instead of 23.4 (5.35 TB/s of algorithmic bytes, 0.82 of
+// the copy bandwidth), a BF16 one at 384^3 64 instead of 74. Holding the
+// registers to 10, 11 or 16 CTAs an SM made a 256^3 step 3, 8 and 45 % slower;
+// unrolling the planes gains nothing in FP32 and 2 % in BF16.
+// Element `off` (in bytes, 32 bits: a colour's array is below 4 GB) of an array.
+template <typename T>
+__device__ __forceinline__ const T* at_byte(const T* p, uint32_t off) { return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + off); }
+template <typename T>
+__device__ __forceinline__ T* at_byte(T* p, uint32_t off) { return reinterpret_cast<T*>(reinterpret_cast<char*>(p) + off); }
+
+template <int KIND, bool DOWN, typename T>
+__device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, const T* __restrict__ v, const T* __restrict__ w, float coef, int colour, int z_chunk, const Dims& d, const GhostRule& g) {
+    constexpr int B = static_cast<int>(sizeof(T));
     const int hx = d.nx / 2, q4 = hx / 4;
     const int j = static_cast<int>(bx) * (32 * kVecRows) + static_cast<int>(threadIdx.y * 32 + threadIdx.x);
     const int y = j / q4, k0 = 4 * (j - y * q4);
     if (y >= d.ny) return;
     const int zb = static_cast<int>(bz) * z_chunk, ze = min(zb + z_chunk, d.nz);
     const bool px = g.periodic[0] != 0, py = g.periodic[1] != 0, pz = g.periodic[2] != 0;
-    const float divisor = KIND == KIND_PRESSURE ? 6.0f : 1.0f + 6.0f * coef;
-    const double recip = tb::recip64(divisor);
-    const int hsz = hx * d.ny;
+    const divide::Divisor div = divide::make_divisor(KIND == KIND_PRESSURE ? 6.0f : 1.0f + 6.0f * coef);
+    const float k = KIND == KIND_PRESSURE ? -coef : coef;
+    const int hsz = hx * d.ny * B;  // bytes of a half plane
     // rows y - 1, y + 1 (offsets in the half plane) and their face ghosts
-    const bool gy_lo = !py && y == 0, gy_hi = !py && y == d.ny - 1;
-    const int oy_lo = y > 0 ? -hx : (py ? (d.ny - 1) * hx : 0), oy_hi = y + 1 < d.ny ? hx : (py ? -(d.ny - 1) * hx : 0);
+    const bool gy_lo = !py && y == 0, gy_hi = !py && y == d.ny - 1, y_face = gy_lo || gy_hi;
+    const int oy_lo = B * (y > 0 ? -hx : (py ? (d.ny - 1) * hx : 0)), oy_hi = B * (y + 1 < d.ny ? hx : (py ? -(d.ny - 1) * hx : 0));
     // the extra x neighbour: k0 - 1 (rows whose u cells sit at even x) or
     // k0 + 4 (odd x), wrapped or replaced by a ghost at a face
     const bool gx_lo = !px && k0 == 0, gx_hi = !px && k0 + 4 == hx;
-    const int ox_lo = k0 > 0 ? -1 : (px ? hx - 1 : 0), ox_hi = k0 + 4 < hx ? 4 : (px ? 4 - hx : 3);
-    // x faces: one cell of the thread (cell 0 on rows whose cells sit at even
-    // x, cell 3 on odd ones) takes its x ghost, from its own value in u;
-    // y faces (the whole row) and z faces (the whole plane) sit behind a
-    // branch interior threads skip, rather than selects every thread executes
-    const bool y_face = gy_lo || gy_hi;
-    const int off_up = pz ? -(d.nz - 1) * hsz : 0;  // plane z + 1 from the top plane (itself on a face)
-    const int off_dn = pz ? (d.nz - 1) * hsz : 0;   // plane z - 1 from the bottom plane
-    const auto update = [&](int z, int i, float4 below, float4 cur, float4 above) {
-        const bool s_odd = ((y + z + colour) & 1) != 0;  // this row's cells of u sit at odd x
-        float ext = ld1v(v + i + (s_odd ? ox_hi : ox_lo));
-        float4 c = ld4v(v + i + oy_lo), e = ld4v(v + i + oy_hi);
-        const float4 r = ld4v(w + i);
-        if (s_odd ? gx_hi : gx_lo) ext = tb::ghost(g, s_odd ? XP : XM, ld1v(u + i + (s_odd ? 3 : 0)));
-        float4 zm = below, zp = above;
-        const bool z_lo = !pz && z == 0, z_hi = !pz && z == d.nz - 1;
+    const int ox_lo = B * (k0 > 0 ? -1 : (px ? hx - 1 : 0)), ox_hi = B * (k0 + 4 < hx ? 4 : (px ? 4 - hx : 3));
+    const float gk_lo = g.k[XM], gk_hi = g.k[XP];
+    const int gm_lo = g.mode[XM], gm_hi = g.mode[XP];
+    // One plane: `near` the plane on the side the march comes from, `cur`; loads
+    // the far one (at offset `far`) and returns it. x faces: one cell of the
+    // thread (cell 0 on rows whose cells sit at even x, cell 3 on odd ones)
+    // takes its x ghost, from its own value in u; y faces (the whole row) and z
+    // faces (the whole plane) sit behind a branch interior threads skip.
+    const auto plane = [&](uint32_t i, bool odd, bool z_lo, bool z_hi, float4 near, float4 cur, int far) {
+        const float4 next = ld4v(at_byte(v, i + far));
+        float ext = ld1v(at_byte(v, i + (odd ? ox_hi : ox_lo)));
+        float4 c = ld4v(at_byte(v, i + oy_lo)), e = ld4v(at_byte(v, i + oy_hi));
+        const float4 r = ld4v(at_byte(w, i));
+        const bool gx = odd ? gx_hi : gx_lo;
+        float self_x = 0.0f;
+        if (gx) self_x = ld1v(at_byte(u, i + (odd ? 3 * B : 0)));
+        float4 zm = DOWN ? next : near, zp = DOWN ? near : next;
         if (y_face || z_lo || z_hi) [[unlikely]] {
-            const float4 self = ld4v(u + i);
+            const float4 self = ld4v(at_byte(u, i));
             if (gy_lo) c = ghost4(g, YM, self);
             if (gy_hi) e = ghost4(g, YP, self);
             if (z_lo) zm = ghost4(g, ZM, self);
             if (z_hi) zp = ghost4(g, ZP, self);
         }
-        const float xm0 = s_odd ? cur.x : ext, xm1 = s_odd ? cur.y : cur.x, xm2 = s_odd ? cur.z : cur.y, xm3 = s_odd ? cur.w : cur.z;
-        const float xp0 = s_odd ? cur.y : cur.x, xp1 = s_odd ? cur.z : cur.y, xp2 = s_odd ? cur.w : cur.z, xp3 = s_odd ? ext : cur.w;
-        float4 o;
-        o.x = vec_update<KIND>(xm0 + xp0 + c.x + e.x + zm.x + zp.x, r.x, coef, divisor, recip);
-        o.y = vec_update<KIND>(xm1 + xp1 + c.y + e.y + zm.y + zp.y, r.y, coef, divisor, recip);
-        o.z = vec_update<KIND>(xm2 + xp2 + c.z + e.z + zm.z + zp.z, r.z, coef, divisor, recip);
-        o.w = vec_update<KIND>(xm3 + xp3 + c.w + e.w + zm.w + zp.w, r.w, coef, divisor, recip);
-        st4v(u + i, o);
+        if (gx) {
+            const int m = odd ? gm_hi : gm_lo;
+            const float q = odd ? gk_hi : gk_lo;
+            ext = m == GHOST_COPY ? self_x : (m == GHOST_CONST ? q : q - self_x);
+        }
+        // x- + x+: the pairs of neighbouring cells of the other colour's row
+        const float p0 = cur.x + cur.y, p1 = cur.y + cur.z, p2 = cur.z + cur.w, pe = ext + (odd ? cur.w : cur.x);
+        float4 n;
+        n.x = (odd ? p0 : pe) + c.x + e.x + zm.x + zp.x;
+        n.y = (odd ? p1 : p0) + c.y + e.y + zm.y + zp.y;
+        n.z = (odd ? p2 : p1) + c.z + e.z + zm.z + zp.z;
+        n.w = (odd ? pe : p2) + c.w + e.w + zm.w + zp.w;
+        // nb - h^2 div, or b + alpha nb, each in one rounding
+        if constexpr (KIND == KIND_PRESSURE) n = make_float4(__fmaf_rn(k, r.x, n.x), __fmaf_rn(k, r.y, n.y), __fmaf_rn(k, r.z, n.z), __fmaf_rn(k, r.w, n.w));
+        else n = make_float4(__fmaf_rn(k, n.x, r.x), __fmaf_rn(k, n.y, r.y), __fmaf_rn(k, n.z, r.z), __fmaf_rn(k, n.w, r.w));
+        constexpr bool six = KIND == KIND_PRESSURE;
+        st4v(at_byte(u, i), make_float4(divide::quotient<six>(n.x, div), divide::quotient<six>(n.y, div), divide::quotient<six>(n.z, div), divide::quotient<six>(n.w, div)));
+        if (!divide::easy(n, div)) [[unlikely]] st4v(at_byte(u, i), divide::hard(n, div));
+        return next;
     };
+    const uint32_t row = static_cast<uint32_t>(B) * static_cast<uint32_t>(k0 + hx * y);
     // DOWN marches the chunk from its top plane (see jacobi_vec4_block)
-    if (!down) {
-        int i = k0 + hx * (y + d.ny * zb);
-        float4 cur = ld4v(v + i);
-        float4 below = ld4v(v + i + (zb > 0 ? -hsz : off_dn));
-        for (int z = zb; z < ze; ++z, i += hsz) {
-            const float4 above = ld4v(v + i + (z + 1 < d.nz ? hsz : off_up));
-            update(z, i, below, cur, above);
-            below = cur;
-            cur = above;
-        }
-    } else {
-        int i = k0 + hx * (y + d.ny * (ze - 1));
-        float4 cur = ld4v(v + i);
-        float4 above = ld4v(v + i + (ze < d.nz ? hsz : off_up));
-        for (int z = ze - 1; z >= zb; --z, i -= hsz) {
-            const float4 below = ld4v(v + i + (z > 0 ? -hsz : off_dn));
-            update(z, i, below, cur, above);
-            above = cur;
-            cur = below;
-        }
+    const int z_first = DOWN ? ze - 1 : zb, step = DOWN ? -hsz : hsz;
+    const int wrap = pz ? (d.nz - 1) * hsz : 0;  // from the bottom plane to the top one (itself on a face)
+    uint32_t i = row + static_cast<uint32_t>(z_first) * static_cast<uint32_t>(hsz);
+    float4 cur = ld4v(at_byte(v, i));
+    float4 near = ld4v(at_byte(v, i + (DOWN ? (ze < d.nz ? hsz : -wrap) : (zb > 0 ? -hsz : wrap))));
+    bool odd = ((y + z_first + colour) & 1) != 0;
+#pragma unroll(sizeof(T) == 2 ? 2 : 1)
+    for (int z = z_first; DOWN ? z >= zb : z < ze; z += DOWN ? -1 : 1, i += step, odd = !odd) {
+        const bool bottom = z == 0, top = z == d.nz - 1;
+        const float4 next = plane(i, odd, !pz && bottom, !pz && top, near, cur, DOWN ? (bottom ? wrap : -hsz) : (top ? -wrap : hsz));
+        near = cur;
+        cur = next;
     }
 }
 
-template <int KIND, typename T>
-__global__ void __launch_bounds__(32 * kVecRows) k_rb_half(T* u, const T* __restrict__ v, const T* __restrict__ w, float coef, int colour, int z_chunk, Dims d, GhostRule g, int down) {
+template <int KIND, bool DOWN, typename T>
+__global__ void __launch_bounds__(32 * kVecRows) k_rb_half(T* u, const T* __restrict__ v, const T* __restrict__ w, float coef, int colour, int z_chunk, Dims d, GhostRule g) {
     wait_for_previous_grid();
-    rb_half_block<KIND, T>(blockIdx.x, blockIdx.z, u, v, w, coef, colour, z_chunk, d, g, down != 0);
+    rb_half_block<KIND, DOWN, T>(blockIdx.x, blockIdx.z, u, v, w, coef, colour, z_chunk, d, g);
 }
 
 // Launch shape of the vectorised kernels: as many z chunks as fit the
@@ -893,13 +919,12 @@ cudaError_t run_rb_split(const StencilArgs& a, cudaStream_t s) {
         ++kernels;
     }
     const GhostRule g = ghost_rule(KIND, a.flow, a.scalar);
-    const auto kern = k_rb_half<KIND, T>;
-    const VecShape vs = plane_shape(d, kern, static_cast<long long>(d.nx / 8) * d.ny);
+    const VecShape vs = plane_shape(d, k_rb_half<KIND, true, T>, static_cast<long long>(d.nx / 8) * d.ny);
     // the two colours march their z chunks in opposite directions, so each
     // launch starts on the planes the one before wrote last (still in L2)
     for (int it = 0; it < a.iterations; ++it) {
-        if ((e = launch_sweep(kern, vs.grid, dim3(32, kVecRows), s, xr, static_cast<const T*>(xb), static_cast<const T*>(br), a.coef, 0, vs.z_chunk, d, g, 0)) != cudaSuccess) return e;
-        if ((e = launch_sweep(kern, vs.grid, dim3(32, kVecRows), s, xb, static_cast<const T*>(xr), static_cast<const T*>(bb), a.coef, 1, vs.z_chunk, d, g, 1)) != cudaSuccess) return e;
+        if ((e = launch_sweep(k_rb_half<KIND, false, T>, vs.grid, dim3(32, kVecRows), s, xr, static_cast<const T*>(xb), static_cast<const T*>(br), a.coef, 0, vs.z_chunk, d, g)) != cudaSuccess) return e;
+        if ((e = launch_sweep(k_rb_half<KIND, true, T>, vs.grid, dim3(32, kVecRows), s, xb, static_cast<const T*>(xr), static_cast<const T*>(bb), a.coef, 1, vs.z_chunk, d, g)) != cudaSuccess) return e;
     }
     if ((e = launch_rb_layout<false, T>(x, xr, xb, nullptr, nullptr, a.out_scale, d, s)) != cudaSuccess) return e;
     if (a.launches) *a.launches += 2 * a.iterations + kernels;
@@ -1345,7 +1370,7 @@ __global__ void __launch_bounds__(32 * kVecRows) k_batch_rb_half(BatchTable t, i
         float* const xb = m.scratch + half;
         const float* const br = m.scratch2;
         const float* const bb = m.scratch2 + half;
-        rb_half_block<KIND, float>(local % bxy, local / bxy, colour ? xb : xr, colour ? xr : xb, colour ? bb : br, coef, colour, m.z_chunk, m.d, m.ghost[KIND]);
+        rb_half_block<KIND, false, float>(local % bxy, local / bxy, colour ? xb : xr, colour ? xr : xb, colour ? bb : br, coef, colour, m.z_chunk, m.d, m.ghost[KIND]);
     }
 }
 

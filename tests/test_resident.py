@@ -67,13 +67,38 @@ def test_resident_solve_of_a_diverged_field(sf, lib, orc, cuda):
     got = []
     for make in (lambda: sf.Simulation(scene.config, scene.scalars, scene.vectors, lib=lib), lambda: orc.Oracle(scene.config, scene.scalars, scene.vectors, precision=32)):
         s = make()
-        s.set_scalar(1, b) if hasattr(s, "set_scalar") else None
+        s.set_scalar(1, b)
         s.step(1)
         got.append(s.fetch(sf.VIEW_SCALAR_FIELD_DATA, 1) if hasattr(s, "ctx") else s.get(orc.SCALAR, 1))
         s.close()
     assert np.array_equal(np.isfinite(got[0]), np.isfinite(got[1]))
     m = np.isfinite(got[0])
     assert m.any() and not m.all() and np.array_equal(got[0][m], got[1][m])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(32, 24, 20), (104, 80, 66)], ids=["resident", "split layout"])
+def test_quotients_over_the_whole_range(n, sf, lib, orc, cuda):
+    """The FP32 quotient and the FP64 one behind it meet in one row: values from
+    the subnormals to the largest, zeros, infinities and NaN, bit for bit the
+    oracle's wherever that is finite."""
+    scene = _scene(sf, n, "stam")
+    rng = np.random.default_rng(1)
+    shape = n[::-1]
+    exponent = rng.integers(-149, 127, (shape[0], shape[1] // 4, 1)).repeat(4, axis=1)
+    b = np.ldexp(rng.standard_normal(shape), exponent).astype(np.float32)
+    b[: shape[0] // 4][rng.random((shape[0] // 4,) + shape[1:]) < 0.7] = 0
+    b[-2, 3, 5], b[-3, 11, 12] = np.inf, np.nan
+    got = []
+    for make in (lambda: sf.Simulation(scene.config, scene.scalars, scene.vectors, lib=lib), lambda: orc.Oracle(scene.config, scene.scalars, scene.vectors, precision=32)):
+        s = make()
+        s.set_scalar(1, b)
+        s.step(1)
+        got.append(s.fetch(sf.VIEW_SCALAR_FIELD_DATA, 1) if hasattr(s, "ctx") else s.get(orc.SCALAR, 1))
+        s.close()
+    m = np.isfinite(got[1])
+    assert m.any() and not m.all() and np.array_equal(np.isfinite(got[0]), m)
+    assert np.array_equal(got[0][m], got[1][m])
 
 
 def test_one_correction_divides_by_six(tmp_path):

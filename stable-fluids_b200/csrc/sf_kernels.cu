@@ -365,8 +365,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_post_diagnostics(float* __restrict__ div, float* __restrict__ mag, const T* __restrict__ vx, const T* __restrict__ vy, const T* __restrict__ vz, Dims d, float h, FlowBC b) { post_diagnostics_block<T>(blockIdx, div, mag, vx, vy, vz, d, h, b); }
 
 // ------------------------------------- divergence / |u| on the z-march --
-// The same values as divergence_block / post_diagnostics_block for FP32
-// fields with nx % 4 == 0: a thread owns one float4 of a row and marches a z
+// The same values as divergence_block / post_diagnostics_block for fields
+// with nx % 4 == 0: a thread owns four cells of a row and marches a z
 // chunk, keeping the z component's planes below / at / above in registers;
 // face ghosts come from the velocity components' GhostRules (copy for
 // outflow and tangential free slip, reflection about the wall velocity
@@ -375,6 +375,10 @@ __global__ void __launch_bounds__(256) k_post_diagnostics(float* __restrict__ di
 // (dz * c) + ((dx * c) + (dy * c)) with the last two sums fused, and
 // |u| = sqrt(w w + (u u + v v)) with the same fusing -- the contraction the
 // reference's expressions take (backend-cuda.cu:391-395, 429-433).
+//
+// The loads bound it: at 384^3 in BF16 (566 MB) it takes 151 us, and 182 with
+// the magnitude; one cell a thread took 516 and 546 (six 2-byte loads a cell,
+// each with its own address and boundary test). FP32 at 256^3: 49 and 60 us.
 constexpr int kDivRows = 4;
 
 struct VelocityGhosts {
@@ -382,6 +386,10 @@ struct VelocityGhosts {
 };
 
 __device__ __forceinline__ float4 ld4f(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ld4f(const __nv_bfloat16* p) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xffff0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xffff0000u));
+}
 __device__ __forceinline__ float4 ghost4f(const GhostRule& g, int face, float4 s) {
     return make_float4(tb::ghost(g, face, s.x), tb::ghost(g, face, s.y), tb::ghost(g, face, s.z), tb::ghost(g, face, s.w));
 }
@@ -390,8 +398,8 @@ __device__ __forceinline__ float magnitude(float u, float v, float w) { return _
 
 // Block `blk` of the launch (blockIdx for one simulation, the work item's
 // block in a batch).
-template <bool MAG>
-__device__ __forceinline__ void divergence_vec4_block(uint3 blk, float* __restrict__ div, float* __restrict__ mag, const float* __restrict__ vx, const float* __restrict__ vy, const float* __restrict__ vz, int z_chunk, const Dims& d, float inv_2h, const GhostRule& gx, const GhostRule& gy, const GhostRule& gz) {
+template <bool MAG, typename T>
+__device__ __forceinline__ void divergence_vec4_block(uint3 blk, float* __restrict__ div, float* __restrict__ mag, const T* __restrict__ vx, const T* __restrict__ vy, const T* __restrict__ vz, int z_chunk, const Dims& d, float inv_2h, const GhostRule& gx, const GhostRule& gy, const GhostRule& gz) {
     const int x0 = 4 * static_cast<int>(blk.x * 32 + threadIdx.x), y = static_cast<int>(blk.y * kDivRows + threadIdx.y);
     if (x0 >= d.nx || y >= d.ny) return;
     const int zb = static_cast<int>(blk.z) * z_chunk, ze = min(zb + z_chunk, d.nz);
@@ -403,8 +411,8 @@ __device__ __forceinline__ void divergence_vec4_block(uint3 blk, float* __restri
     for (int z = zb; z < ze; ++z, i += sz) {
         const float4 zhi = z + 1 < d.nz ? ld4f(vz + i + sz) : (pz ? ld4f(vz + i - (d.nz - 1) * sz) : ghost4f(gz, ZP, zc));
         const float4 xc = ld4f(vx + i);
-        const float xl = x0 > 0 ? vx[i - 1] : (px ? vx[i + d.nx - 1] : tb::ghost(gx, XM, xc.x));
-        const float xr = x0 + 4 < d.nx ? vx[i + 4] : (px ? vx[i + 4 - d.nx] : tb::ghost(gx, XP, xc.w));
+        const float xl = x0 > 0 ? to_f(vx[i - 1]) : (px ? to_f(vx[i + d.nx - 1]) : tb::ghost(gx, XM, xc.x));
+        const float xr = x0 + 4 < d.nx ? to_f(vx[i + 4]) : (px ? to_f(vx[i + 4 - d.nx]) : tb::ghost(gx, XP, xc.w));
         const float4 yc = ld4f(vy + i);
         const float4 ylo = y > 0 ? ld4f(vy + i - sy) : (py ? ld4f(vy + i + (d.ny - 1) * sy) : ghost4f(gy, YM, yc));
         const float4 yhi = y + 1 < d.ny ? ld4f(vy + i + sy) : (py ? ld4f(vy + i - (d.ny - 1) * sy) : ghost4f(gy, YP, yc));
@@ -420,9 +428,9 @@ __device__ __forceinline__ void divergence_vec4_block(uint3 blk, float* __restri
     }
 }
 
-template <bool MAG>
-__global__ void __launch_bounds__(32 * kDivRows) k_divergence_vec4(float* __restrict__ div, float* __restrict__ mag, const float* __restrict__ vx, const float* __restrict__ vy, const float* __restrict__ vz, int z_chunk, Dims d, float inv_2h, VelocityGhosts gh) {
-    divergence_vec4_block<MAG>(blockIdx, div, mag, vx, vy, vz, z_chunk, d, inv_2h, gh.g[0], gh.g[1], gh.g[2]);
+template <bool MAG, typename T>
+__global__ void __launch_bounds__(32 * kDivRows) k_divergence_vec4(float* __restrict__ div, float* __restrict__ mag, const T* __restrict__ vx, const T* __restrict__ vy, const T* __restrict__ vz, int z_chunk, Dims d, float inv_2h, VelocityGhosts gh) {
+    divergence_vec4_block<MAG, T>(blockIdx, div, mag, vx, vy, vz, z_chunk, d, inv_2h, gh.g[0], gh.g[1], gh.g[2]);
 }
 
 // ------------------------------------------------------- work-table batch --
@@ -602,9 +610,10 @@ cudaError_t launch_scale(void* data, float factor, size_t n, int bf16, cudaStrea
 
 GhostRule make_ghost_rule(int kind, const FlowBC& fb, const ScalarBC& sb);
 
-// The z-marching divergence for FP32 fields whose rows are whole float4s:
+// The z-marching divergence for fields whose rows are whole groups of four:
 // false (nothing launched) when the grid or the pointers do not suit it.
-bool launch_divergence_vec4(float* div, float* mag, const void* vx, const void* vy, const void* vz, Dims d, float h, const FlowBC& b, cudaStream_t s) {
+template <typename T>
+bool launch_divergence_vec4(float* div, float* mag, const T* vx, const T* vy, const T* vz, Dims d, float h, const FlowBC& b, cudaStream_t s) {
     const auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     const size_t cells = static_cast<size_t>(d.nx) * d.ny * d.nz;
     if (d.nx % 4 != 0 || cells >= (1ull << 31) || !al(div) || !al(vx) || !al(vy) || !al(vz) || (mag != nullptr && !al(mag))) return false;
@@ -612,7 +621,7 @@ bool launch_divergence_vec4(float* div, float* mag, const void* vx, const void* 
     for (int c = 0; c < 3; ++c) gh.g[c] = make_ghost_rule(KIND_VEL_X + c, b, ScalarBC{});
     static int per_sm = [] {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_divergence_vec4<true>, 32 * kDivRows, 0) != cudaSuccess || n < 1) n = 8;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_divergence_vec4<true, T>, 32 * kDivRows, 0) != cudaSuccess || n < 1) n = 8;
         return n;
     }();
     int sms = 148, dev = 0;
@@ -624,13 +633,18 @@ bool launch_divergence_vec4(float* div, float* mag, const void* vx, const void* 
     if (z_chunk < 4) z_chunk = d.nz < 4 ? d.nz : 4;
     const dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(by), static_cast<unsigned>((d.nz + z_chunk - 1) / z_chunk));
     const float inv_2h = 0.5f / h;
-    if (mag) k_divergence_vec4<true><<<grid, dim3(32, kDivRows), 0, s>>>(div, mag, static_cast<const float*>(vx), static_cast<const float*>(vy), static_cast<const float*>(vz), z_chunk, d, inv_2h, gh);
-    else k_divergence_vec4<false><<<grid, dim3(32, kDivRows), 0, s>>>(div, nullptr, static_cast<const float*>(vx), static_cast<const float*>(vy), static_cast<const float*>(vz), z_chunk, d, inv_2h, gh);
+    if (mag) k_divergence_vec4<true, T><<<grid, dim3(32, kDivRows), 0, s>>>(div, mag, vx, vy, vz, z_chunk, d, inv_2h, gh);
+    else k_divergence_vec4<false, T><<<grid, dim3(32, kDivRows), 0, s>>>(div, nullptr, vx, vy, vz, z_chunk, d, inv_2h, gh);
     return true;
 }
 
+bool launch_divergence_vec4(float* div, float* mag, const void* vx, const void* vy, const void* vz, Dims d, float h, const FlowBC& b, int bf16, cudaStream_t s) {
+    if (bf16) return launch_divergence_vec4(div, mag, static_cast<const bf16_t*>(vx), static_cast<const bf16_t*>(vy), static_cast<const bf16_t*>(vz), d, h, b, s);
+    return launch_divergence_vec4(div, mag, static_cast<const float*>(vx), static_cast<const float*>(vy), static_cast<const float*>(vz), d, h, b, s);
+}
+
 cudaError_t launch_divergence(float* div, const void* vx, const void* vy, const void* vz, Dims d, float h, const FlowBC& b, int bf16, cudaStream_t s) {
-    if (!bf16 && launch_divergence_vec4(div, nullptr, vx, vy, vz, d, h, b, s)) return cudaGetLastError();
+    if (launch_divergence_vec4(div, nullptr, vx, vy, vz, d, h, b, bf16, s)) return cudaGetLastError();
     SFB_STORAGE(bf16, (k_divergence<float><<<cell_grid(d), cell_block(), 0, s>>>(div, static_cast<const float*>(vx), static_cast<const float*>(vy), static_cast<const float*>(vz), d, h, b)),
                 (k_divergence<bf16_t><<<cell_grid(d), cell_block(), 0, s>>>(div, static_cast<const bf16_t*>(vx), static_cast<const bf16_t*>(vy), static_cast<const bf16_t*>(vz), d, h, b)));
     return cudaGetLastError();
@@ -668,7 +682,7 @@ cudaError_t launch_warm_start_select(DeviceStats* learned, const DeviceStats* pl
 }
 
 cudaError_t launch_post_diagnostics(float* div, float* mag, const void* vx, const void* vy, const void* vz, Dims d, float h, const FlowBC& b, int bf16, cudaStream_t s) {
-    if (!bf16 && launch_divergence_vec4(div, mag, vx, vy, vz, d, h, b, s)) return cudaGetLastError();
+    if (launch_divergence_vec4(div, mag, vx, vy, vz, d, h, b, bf16, s)) return cudaGetLastError();
     SFB_STORAGE(bf16, (k_post_diagnostics<float><<<cell_grid(d), cell_block(), 0, s>>>(div, mag, static_cast<const float*>(vx), static_cast<const float*>(vy), static_cast<const float*>(vz), d, h, b)),
                 (k_post_diagnostics<bf16_t><<<cell_grid(d), cell_block(), 0, s>>>(div, mag, static_cast<const bf16_t*>(vx), static_cast<const bf16_t*>(vy), static_cast<const bf16_t*>(vz), d, h, b)));
     return cudaGetLastError();

@@ -549,9 +549,15 @@ __global__ void __launch_bounds__(256) k_rb_layout(T* __restrict__ field, T* __r
 // With 32-bit byte offsets, the FP32 quotient and its test after the store
 // (divide::easy; a branch before the store would hold it back), a colour at
 // 256^3 takes 18.8 us instead of 23.4 (5.35 TB/s of algorithmic bytes, 0.82 of
-// the copy bandwidth), a BF16 one at 384^3 64 instead of 74. Holding the
-// registers to 10, 11 or 16 CTAs an SM made a 256^3 step 3, 8 and 45 % slower;
-// unrolling the planes gains nothing in FP32 and 2 % in BF16.
+// the copy bandwidth), at 384^3 64 instead of 74. BF16 moves half the bytes and
+// stays bound by issue (0.69 of the slots): there the sums and quotients go in
+// packed pairs, and a diffusion's colour at 384^3 takes 53 us instead of 71
+// (57 without the pairs; pairs in FP32 gain 1 % in the diffusion and cost 2 % in
+// the pressure). Slower, all measured: the registers held to 10, 11 or 16 CTAs
+// an SM (3, 8 and 45 %), planes unrolled by 2 to 4 (4 % in BF16, up to 6 % in
+// FP32), a plane's loads one plane ahead (8 %), eight BF16 cells a thread (13 %,
+// at most 24 warps an SM), and planes brought to shared memory by bulk copies
+// (36 %: a third more instructions).
 // Element `off` (in bytes, 32 bits: a colour's array is below 4 GB) of an array.
 template <typename T>
 __device__ __forceinline__ const T* at_byte(const T* p, uint32_t off) { return reinterpret_cast<const T*>(reinterpret_cast<const char*>(p) + off); }
@@ -607,16 +613,25 @@ __device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, co
         }
         // x- + x+: the pairs of neighbouring cells of the other colour's row
         const float p0 = cur.x + cur.y, p1 = cur.y + cur.z, p2 = cur.z + cur.w, pe = ext + (odd ? cur.w : cur.x);
-        float4 n;
-        n.x = (odd ? p0 : pe) + c.x + e.x + zm.x + zp.x;
-        n.y = (odd ? p1 : p0) + c.y + e.y + zm.y + zp.y;
-        n.z = (odd ? p2 : p1) + c.z + e.z + zm.z + zp.z;
-        n.w = (odd ? pe : p2) + c.w + e.w + zm.w + zp.w;
-        // nb - h^2 div, or b + alpha nb, each in one rounding
-        if constexpr (KIND == KIND_PRESSURE) n = make_float4(__fmaf_rn(k, r.x, n.x), __fmaf_rn(k, r.y, n.y), __fmaf_rn(k, r.z, n.z), __fmaf_rn(k, r.w, n.w));
-        else n = make_float4(__fmaf_rn(k, n.x, r.x), __fmaf_rn(k, n.y, r.y), __fmaf_rn(k, n.z, r.z), __fmaf_rn(k, n.w, r.w));
+        const float4 x = make_float4(odd ? p0 : pe, odd ? p1 : p0, odd ? p2 : p1, odd ? pe : p2);
         constexpr bool six = KIND == KIND_PRESSURE;
-        st4v(at_byte(u, i), make_float4(divide::quotient<six>(n.x, div), divide::quotient<six>(n.y, div), divide::quotient<six>(n.z, div), divide::quotient<six>(n.w, div)));
+        float4 n, o;
+        // nb - h^2 div, or b + alpha nb, each in one rounding, then the quotient
+        if constexpr (sizeof(T) == 2) {  // in pairs
+            const F2 k2 = f2(k, k);
+            F4 m = f4(x) + f4(c) + f4(e) + f4(zm) + f4(zp);
+            const F4 b = f4(r);
+            if constexpr (six) m = {fma2(k2, b.lo, m.lo), fma2(k2, b.hi, m.hi)};
+            else m = {fma2(k2, m.lo, b.lo), fma2(k2, m.hi, b.hi)};
+            n = unpack(m);
+            o = unpack(F4{divide::quotient<six>(m.lo, div), divide::quotient<six>(m.hi, div)});
+        } else {
+            n = make_float4(x.x + c.x + e.x + zm.x + zp.x, x.y + c.y + e.y + zm.y + zp.y, x.z + c.z + e.z + zm.z + zp.z, x.w + c.w + e.w + zm.w + zp.w);
+            if constexpr (six) n = make_float4(__fmaf_rn(k, r.x, n.x), __fmaf_rn(k, r.y, n.y), __fmaf_rn(k, r.z, n.z), __fmaf_rn(k, r.w, n.w));
+            else n = make_float4(__fmaf_rn(k, n.x, r.x), __fmaf_rn(k, n.y, r.y), __fmaf_rn(k, n.z, r.z), __fmaf_rn(k, n.w, r.w));
+            o = make_float4(divide::quotient<six>(n.x, div), divide::quotient<six>(n.y, div), divide::quotient<six>(n.z, div), divide::quotient<six>(n.w, div));
+        }
+        st4v(at_byte(u, i), o);
         if (!divide::easy(n, div)) [[unlikely]] st4v(at_byte(u, i), divide::hard(n, div));
         return next;
     };
@@ -628,7 +643,7 @@ __device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, co
     float4 cur = ld4v(at_byte(v, i));
     float4 near = ld4v(at_byte(v, i + (DOWN ? (ze < d.nz ? hsz : -wrap) : (zb > 0 ? -hsz : wrap))));
     bool odd = ((y + z_first + colour) & 1) != 0;
-#pragma unroll(sizeof(T) == 2 ? 2 : 1)
+#pragma unroll 1
     for (int z = z_first; DOWN ? z >= zb : z < ze; z += DOWN ? -1 : 1, i += step, odd = !odd) {
         const bool bottom = z == 0, top = z == d.nz - 1;
         const float4 next = plane(i, odd, !pz && bottom, !pz && top, near, cur, DOWN ? (bottom ? wrap : -hsz) : (top ? -wrap : hsz));

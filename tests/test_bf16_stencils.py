@@ -40,3 +40,32 @@ def test_divergence_and_magnitude_of_bf16_velocity(n, periodic_z, sf, lib, cuda)
     assert top > 0
     assert np.abs(div - want).max() <= 3 * 4 * 2.0**-24 * 2 * top / (2 * h)
     assert np.abs(mag - np.sqrt((u**2).sum(0))).max() <= 4 * 2.0**-24 * np.sqrt(3) * top
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(104, 80, 66), (8, 300, 240)], ids=lambda n: "x".join(map(str, n)))
+def test_bf16_half_sweeps_over_the_whole_range(n, sf, lib, cuda):
+    """The split layout's packed sums and quotients give the colour launches'
+    bits (iterations_per_pass 1) from the subnormals to the largest values,
+    zeros and infinities among them."""
+    rng = np.random.default_rng(2)
+    shape = n[::-1]
+    exponent = rng.integers(-133, 126, (shape[0], shape[1] // 4, 1)).repeat(4, axis=1)
+    with np.errstate(over="ignore"):
+        b = np.ldexp(rng.standard_normal(shape), exponent).astype(np.float32)
+    b[: shape[0] // 4][rng.random((shape[0] // 4,) + shape[1:]) < 0.7] = 0
+    b[-2, 3, 5] = np.inf
+    scene = sf.scenes.plume("bf16", n, diffuse_iterations=3, pressure_iterations=2, walls=sf.scenes.stam_walls(), velocity_seed=3, steps=1)
+    got = []
+    for per_pass in (0, 1):
+        o = sf.default_options(lib)
+        o.storage, o.iterations_per_pass = sf.STORAGE_BF16, per_pass
+        sim = sf.Simulation(scene.config, scene.scalars, scene.vectors, lib=lib, options=o)
+        sim.set_scalar(1, b)
+        sim.step(1)
+        got.append([sim.fetch(sf.VIEW_SCALAR_FIELD_DATA, 1), *sim.fetch(sf.VIEW_FLOW_VELOCITY)])
+        sim.close()
+    for a, c in zip(*got):
+        m = np.isfinite(c)
+        assert m.any() and np.array_equal(np.isfinite(a), m) and np.array_equal(a[m], c[m])
+    assert not np.isfinite(got[0][0]).all()

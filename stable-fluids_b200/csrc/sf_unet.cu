@@ -41,6 +41,9 @@ unsigned blocks_for(size_t n) {
     return static_cast<unsigned>(b < 148u * 32u ? (b == 0 ? 1 : b) : 148u * 32u);
 }
 
+// Blocks of a kernel that ends in one atomic a block.
+unsigned sum_blocks(size_t n) { return std::min(blocks_for(n), 148u * 8u); }
+
 struct Layer {
     int cin, cout;  // padded channel counts
     int cin_real;   // channels carrying data (fan-in of the initialisation)
@@ -402,12 +405,12 @@ float* GB(Net* n, int l) { return n->g + n->layers[l].off + n->layers[l].wn; }
     } while (0)
 
 // Forward pass from b (scaled inside) and p_prev; leaves the FP32 output in
-// buf->out and every activation in place for the backward pass. 20 kernels.
+// buf->out and every activation in place for the backward pass. 18 kernels.
 cudaError_t forward(Net* n, const float* b, float b_factor, const float* p_prev, cudaStream_t s) {
     Buffers& B = *n->buf;
     cudaError_t e;
     SFB_TRY(cudaMemsetAsync(B.sums, 0, sizeof(double), s));
-    k_sum_squares<<<blocks_for(B.n0), 256, 0, s>>>(b, b_factor, B.n0, B.sums);
+    k_sum_squares<<<sum_blocks(B.n0), 256, 0, s>>>(b, b_factor, B.n0, B.sums);
     k_finish_scale<<<1, 32, 0, s>>>(B.sums, static_cast<double>(B.n0), B.scale);
     k_pack_input<<<blocks_for(B.n0), 256, 0, s>>>(b, p_prev, B.scale, b_factor, B.in, B.n0);
     SFB_TRY(cudaGetLastError());
@@ -419,12 +422,10 @@ cudaError_t forward(Net* n, const float* b, float b_factor, const float* p_prev,
     k_pool2<<<row_grid(B.d2.nx, 4, B.d2.ny, B.d2.nz), 256, 0, s>>>(B.e1b, 32, 0, B.p1, 32, B.d2);
     SFB_TRY(conv_any(32, 64, tc::RELU_BF16, B.p1, W(n, BA), Bias(n, BA), B.ba, 64, 0, B.d2, s, n->error));
     SFB_TRY(conv_any(64, 64, tc::RELU_BF16, B.ba, W(n, BB), Bias(n, BB), B.bb, 64, 0, B.d2, s, n->error));
-    k_upsample2<<<row_grid(B.d1.nx, 8, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.bb, 64, B.d2, B.cat1, 96, 0);
-    k_copy_channels<<<blocks_for(B.n1 * 4), 256, 0, s>>>(B.e1b, 32, 0, B.cat1, 96, 64, 32, B.n1, 0);
+    k_upsample2_concat<<<row_grid(B.d1.nx, 12, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.bb, 64, B.d2, B.e1b, 32, B.cat1);
     SFB_TRY(conv_any(96, 32, tc::RELU_BF16, B.cat1, W(n, D1A), Bias(n, D1A), B.d1a, 32, 0, B.d1, s, n->error));
     SFB_TRY(conv_any(32, 32, tc::RELU_BF16, B.d1a, W(n, D1B), Bias(n, D1B), B.d1b, 32, 0, B.d1, s, n->error));
-    k_upsample2<<<row_grid(B.d0.nx, 4, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.d1b, 32, B.d1, B.cat0, 48, 0);
-    k_copy_channels<<<blocks_for(B.n0 * 2), 256, 0, s>>>(B.e0b, 16, 0, B.cat0, 48, 32, 16, B.n0, 0);
+    k_upsample2_concat<<<row_grid(B.d0.nx, 6, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.d1b, 32, B.d1, B.e0b, 16, B.cat0);
     SFB_TRY(conv_any(48, 16, tc::RELU_BF16, B.cat0, W(n, D0A), Bias(n, D0A), B.d0a, 16, 0, B.d0, s, n->error));
     SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.d0a, W(n, D0B), Bias(n, D0B), B.d0b, 16, 0, B.d0, s, n->error));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_F32_CH0, B.d0b, W(n, OUT), Bias(n, OUT), B.out, 1, 0, B.d0, s, n->error));
@@ -454,35 +455,29 @@ cudaError_t backward(Net* n, cudaStream_t s) {
     if (chained) chain.add(B.cat0, 48, B.gd0a, GW(n, D0A), GB(n, D0A), static_cast<long long>(B.n0));
     else SFB_TRY(wgrad_any(48, 16, B.cat0, B.gd0a, GW(n, D0A), GB(n, D0A), B.d0, s, n->error));
     SFB_TRY(conv_any(16, 48, tc::LINEAR_BF16, B.gd0a, WT(n, D0A), nullptr, B.gcat0, 48, 0, B.d0, s, n->error));
-    k_upsample2_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat0, 48, 0, 32, B.d1, B.gd1b);
+    k_upsample2_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat0, 48, 0, 32, B.d1, B.d1b, B.gd1b);
     // d1b, d1a (input of d1a: cat1 = [up(bb) | e1b])
-    k_relu_backward<<<blocks_for(B.n1 * 32 / 8), 256, 0, s>>>(B.gd1b, B.d1b, B.n1 * 32);
     SFB_TRY(wgrad_any(32, 32, B.d1a, B.gd1b, GW(n, D1B), GB(n, D1B), B.d1, s, n->error));
     SFB_TRY(conv_any(32, 32, tc::LINEAR_BF16, B.gd1b, WT(n, D1B), nullptr, B.gd1a, 32, 0, B.d1, s, n->error));
     k_relu_backward<<<blocks_for(B.n1 * 32 / 8), 256, 0, s>>>(B.gd1a, B.d1a, B.n1 * 32);
     SFB_TRY(wgrad_any(96, 32, B.cat1, B.gd1a, GW(n, D1A), GB(n, D1A), B.d1, s, n->error));
     SFB_TRY(conv_any(32, 96, tc::LINEAR_BF16, B.gd1a, WT(n, D1A), nullptr, B.gcat1, 96, 0, B.d1, s, n->error));
-    k_upsample2_backward<<<row_grid(B.d2.nx, 8, B.d2.ny, B.d2.nz), 256, 0, s>>>(B.gcat1, 96, 0, 64, B.d2, B.gbb);
+    k_upsample2_backward<<<row_grid(B.d2.nx, 8, B.d2.ny, B.d2.nz), 256, 0, s>>>(B.gcat1, 96, 0, 64, B.d2, B.bb, B.gbb);
     // bottleneck
-    k_relu_backward<<<blocks_for(B.n2 * 64 / 8), 256, 0, s>>>(B.gbb, B.bb, B.n2 * 64);
     SFB_TRY(wgrad_any(64, 64, B.ba, B.gbb, GW(n, BB), GB(n, BB), B.d2, s, n->error));
     SFB_TRY(conv_any(64, 64, tc::LINEAR_BF16, B.gbb, WT(n, BB), nullptr, B.gba, 64, 0, B.d2, s, n->error));
     k_relu_backward<<<blocks_for(B.n2 * 64 / 8), 256, 0, s>>>(B.gba, B.ba, B.n2 * 64);
     SFB_TRY(wgrad_any(32, 64, B.p1, B.gba, GW(n, BA), GB(n, BA), B.d2, s, n->error));
     SFB_TRY(conv_any(64, 32, tc::LINEAR_BF16, B.gba, WT(n, BA), nullptr, B.gp1, 32, 0, B.d2, s, n->error));
     // e1b receives the skip (channels 64..95 of cat1) and the pooled path
-    k_copy_channels<<<blocks_for(B.n1 * 4), 256, 0, s>>>(B.gcat1, 96, 64, B.ge1b, 32, 0, 32, B.n1, 0);
-    k_pool2_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gp1, 32, B.d2, B.ge1b, 32, 0, 1);
-    k_relu_backward<<<blocks_for(B.n1 * 32 / 8), 256, 0, s>>>(B.ge1b, B.e1b, B.n1 * 32);
+    k_skip_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat1, 96, 64, B.e1b, B.gp1, 32, B.d2, B.ge1b);
     SFB_TRY(wgrad_any(32, 32, B.e1a, B.ge1b, GW(n, E1B), GB(n, E1B), B.d1, s, n->error));
     SFB_TRY(conv_any(32, 32, tc::LINEAR_BF16, B.ge1b, WT(n, E1B), nullptr, B.ge1a, 32, 0, B.d1, s, n->error));
     k_relu_backward<<<blocks_for(B.n1 * 32 / 8), 256, 0, s>>>(B.ge1a, B.e1a, B.n1 * 32);
     SFB_TRY(wgrad_any(16, 32, B.p0, B.ge1a, GW(n, E1A), GB(n, E1A), B.d1, s, n->error));
     SFB_TRY(conv_any(32, 16, tc::LINEAR_BF16, B.ge1a, WT(n, E1A), nullptr, B.gp0, 16, 0, B.d1, s, n->error));
     // e0b: skip (channels 32..47 of cat0) + pooled path
-    k_copy_channels<<<blocks_for(B.n0 * 2), 256, 0, s>>>(B.gcat0, 48, 32, B.ge0b, 16, 0, 16, B.n0, 0);
-    k_pool2_backward<<<row_grid(B.d0.nx, 2, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.gp0, 16, B.d1, B.ge0b, 16, 0, 1);
-    k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.ge0b, B.e0b, B.n0 * 16);
+    k_skip_backward<<<row_grid(B.d0.nx, 2, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.gcat0, 48, 32, B.e0b, B.gp0, 16, B.d1, B.ge0b);
     if (chained) chain.add(B.e0a, 16, B.ge0b, GW(n, E0B), GB(n, E0B), static_cast<long long>(B.n0));
     else SFB_TRY(wgrad_any(16, 16, B.e0a, B.ge0b, GW(n, E0B), GB(n, E0B), B.d0, s, n->error));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.ge0b, WT(n, E0B), nullptr, B.ge0a, 16, 0, B.d0, s, n->error));
@@ -505,7 +500,7 @@ cudaError_t loss_and_gradients(Net* n, const float* b, float b_factor, const flo
     Buffers& B = *n->buf;
     k_make_target<<<blocks_for(B.n0), 256, 0, s>>>(p_target, p_prev, B.scale, B.target, B.n0);
     SFB_TRY(cudaMemsetAsync(B.sums + 1, 0, sizeof(double), s));
-    k_mse<<<blocks_for(B.n0), 256, 0, s>>>(B.out, B.target, B.n0, B.g16, B.sums + 1);
+    k_mse<<<sum_blocks(B.n0), 256, 0, s>>>(B.out, B.target, B.n0, B.g16, B.sums + 1);
     SFB_TRY(backward(n, s));
     double sum = 0.0;
     SFB_TRY(cudaMemcpyAsync(&sum, B.sums + 1, sizeof(double), cudaMemcpyDeviceToHost, s));

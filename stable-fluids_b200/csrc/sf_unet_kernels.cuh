@@ -43,15 +43,28 @@ __global__ void k_finish_scale(const double* __restrict__ sumsq, double n, float
     }
 }
 
-__global__ void k_sum_squares(const float* __restrict__ b, float b_factor, size_t n, double* __restrict__ out) {
+// Adds the block's sum of acc to *out: one atomic a block. (One a warp, of 4736
+// blocks, made the sum over 128^3 voxels wait 62 us for its atomics; now it takes 8.)
+// 256 threads, all of them.
+__device__ __forceinline__ void add_block_sum(double acc, double* out) {
+    __shared__ double part[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) acc += part[k];
+        atomicAdd(out, acc);
+    }
+}
+
+__global__ void __launch_bounds__(256) k_sum_squares(const float* __restrict__ b, float b_factor, size_t n, double* __restrict__ out) {
     double acc = 0.0;
     for (size_t v = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; v < n; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
         const double x = static_cast<double>(b[v]) * b_factor;
         acc += x * x;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, acc);
+    add_block_sum(acc, out);
 }
 
 // p0 = p_prev + delta / scale (the network predicts the scaled correction).
@@ -61,7 +74,7 @@ __global__ void k_unpack_output(const float* __restrict__ delta, const float* p_
     for (size_t v = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; v < n; v += static_cast<size_t>(gridDim.x) * blockDim.x) p0[v] = (p_prev ? p_prev[v] : 0.0f) + delta[v] * inv;
 }
 
-// The pooling / upsampling / copy kernels below move 8 channels (16 bytes)
+// The pooling and upsampling kernels below move 8 channels (16 bytes)
 // per thread; channel counts, strides and offsets are multiples of 8. The
 // 2-D launches give blockIdx.y = y and blockIdx.z = z of the output grid and
 // threads over (x, 8-channel chunk) of one row.
@@ -111,43 +124,55 @@ __global__ void k_pool2(const __nv_bfloat16* __restrict__ in, int in_ch, int in_
     store8(out + v * C + c, s);
 }
 
-// Backward of the pooling: each fine voxel gets 1/8 of its parent's gradient,
-// added to (accumulate) or written into the fine gradient tensor.
-// Launch: row_grid(fine nx, C / 8, fine ny, fine nz).
-__global__ void k_pool2_backward(const __nv_bfloat16* __restrict__ gcoarse, int C, Dims coarse, __nv_bfloat16* __restrict__ gfine, int fine_ch, int fine_off, int accumulate) {
-    const int c8n = C / 8, fnx = coarse.nx * 2, fny = coarse.ny * 2;
-    const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (i >= fnx * c8n) return;
-    const int x = i / c8n, c = (i % c8n) * 8, y = static_cast<int>(blockIdx.y), z = static_cast<int>(blockIdx.z);
-    const size_t cv = static_cast<size_t>(x / 2) + static_cast<size_t>(coarse.nx) * (y / 2 + static_cast<size_t>(coarse.ny) * (z / 2));
-    Bf8 g = load8(gcoarse + cv * C + c);
-    __nv_bfloat16* dst = gfine + (static_cast<size_t>(x) + static_cast<size_t>(fnx) * (y + static_cast<size_t>(fny) * z)) * fine_ch + fine_off + c;
-    const Bf8 old = accumulate ? load8(dst) : Bf8{};
+// The gradient through a ReLU whose output is act.
+__device__ __forceinline__ void relu_mask(Bf8& g, const Bf8& act) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        g.v[j] = 0.125f * g.v[j];
-        if (accumulate) g.v[j] += old.v[j];
-    }
-    store8(dst, g);
+    for (int j = 0; j < 8; ++j)
+        if (!(act.v[j] > 0.0f)) g.v[j] = 0.0f;
 }
 
-// Nearest 2x upsampling of a coarse tensor into channels [out_off, out_off+C)
-// of a fine tensor with channel stride out_ch. Launch: row_grid(fine nx, C / 8,
-// fine ny, fine nz).
-__global__ void k_upsample2(const __nv_bfloat16* __restrict__ in, int C, Dims coarse, __nv_bfloat16* __restrict__ out, int out_ch, int out_off) {
+// Gradient of an encoder level's output, which feeds the skip connection and
+// the pooling: channels [off, off + C) of the concatenation's gradient plus 1/8
+// of the coarse parent's, rounded to BF16, through the ReLU whose output is act (C
+// channels). Launch: row_grid(fine nx, C / 8, fine ny, fine nz). One pass over memory: a copy, an addition and a mask in
+// passes of their own took 86 us at 128^3 with 16 channels, this 48.
+__global__ void k_skip_backward(const __nv_bfloat16* __restrict__ gcat, int cat_ch, int off, const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __restrict__ gcoarse, int C, Dims coarse, __nv_bfloat16* __restrict__ gfine) {
     const int c8n = C / 8, fnx = coarse.nx * 2, fny = coarse.ny * 2;
     const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= fnx * c8n) return;
     const int x = i / c8n, c = (i % c8n) * 8, y = static_cast<int>(blockIdx.y), z = static_cast<int>(blockIdx.z);
     const size_t cv = static_cast<size_t>(x / 2) + static_cast<size_t>(coarse.nx) * (y / 2 + static_cast<size_t>(coarse.ny) * (z / 2));
     const size_t fv = static_cast<size_t>(x) + static_cast<size_t>(fnx) * (y + static_cast<size_t>(fny) * z);
-    *reinterpret_cast<uint4*>(out + fv * out_ch + out_off + c) = *reinterpret_cast<const uint4*>(in + cv * C + c);
+    const Bf8 skip = load8(gcat + fv * cat_ch + off + c), a = load8(act + fv * C + c);
+    Bf8 g = load8(gcoarse + cv * C + c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g.v[j] = __fmaf_rn(0.125f, g.v[j], skip.v[j]);
+    relu_mask(g, a);
+    store8(gfine + fv * C + c, g);
 }
 
-// Backward of the upsampling: the coarse gradient is the sum over its 8
-// children of channels [off, off + C) of the fine gradient. Launch:
-// row_grid(coarse.nx, C / 8, coarse.ny, coarse.nz).
-__global__ void k_upsample2_backward(const __nv_bfloat16* __restrict__ gfine, int fine_ch, int off, int C, Dims coarse, __nv_bfloat16* __restrict__ gcoarse) {
+// The input of a decoder level: the coarse tensor upsampled 2x (nearest) in
+// channels [0, C), the skip connection in the S after them. Launch:
+// row_grid(fine nx, (C + S) / 8, fine ny, fine nz). Bound by its writes (61 us
+// for 272 MB at the finest level of 128^3, as long as the two parts in passes of
+// their own took; one launch less). Convolutions that wrote their channels of
+// the concatenation themselves lost as much as the copy took: 32 bytes of every
+// 96, and the pooling and the backward pass read them so too.
+__global__ void k_upsample2_concat(const __nv_bfloat16* __restrict__ in, int C, Dims coarse, const __nv_bfloat16* __restrict__ skip, int S, __nv_bfloat16* __restrict__ out) {
+    const int c8n = (C + S) / 8, fnx = coarse.nx * 2, fny = coarse.ny * 2;
+    const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= fnx * c8n) return;
+    const int x = i / c8n, c = (i % c8n) * 8, y = static_cast<int>(blockIdx.y), z = static_cast<int>(blockIdx.z);
+    const size_t cv = static_cast<size_t>(x / 2) + static_cast<size_t>(coarse.nx) * (y / 2 + static_cast<size_t>(coarse.ny) * (z / 2));
+    const size_t fv = static_cast<size_t>(x) + static_cast<size_t>(fnx) * (y + static_cast<size_t>(fny) * z);
+    const __nv_bfloat16* const from = c < C ? in + cv * C + c : skip + fv * S + (c - C);
+    *reinterpret_cast<uint4*>(out + fv * (C + S) + c) = *reinterpret_cast<const uint4*>(from);
+}
+
+// Backward of the upsampling and of the ReLU before it (its output act): the
+// coarse gradient is the sum over its 8 children of channels [off, off + C) of
+// the fine gradient. Launch: row_grid(coarse.nx, C / 8, coarse.ny, coarse.nz).
+__global__ void k_upsample2_backward(const __nv_bfloat16* __restrict__ gfine, int fine_ch, int off, int C, Dims coarse, const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ gcoarse) {
     const int c8n = C / 8, fnx = coarse.nx * 2, fny = coarse.ny * 2;
     const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= coarse.nx * c8n) return;
@@ -160,44 +185,23 @@ __global__ void k_upsample2_backward(const __nv_bfloat16* __restrict__ gfine, in
         for (int j = 0; j < 8; ++j) s.v[j] += a.v[j];
     }
     const size_t v = static_cast<size_t>(x) + static_cast<size_t>(coarse.nx) * (y + static_cast<size_t>(coarse.ny) * z);
+    relu_mask(s, load8(act + v * C + c));
     store8(gcoarse + v * C + c, s);
-}
-
-// Copies channels [src_off, src_off + C) of src into [dst_off, ...) of dst
-// (adding to dst when accumulate), 8 channels per thread.
-__global__ void k_copy_channels(const __nv_bfloat16* __restrict__ src, int src_ch, int src_off, __nv_bfloat16* __restrict__ dst, int dst_ch, int dst_off, int C, size_t voxels, int accumulate) {
-    const size_t c8n = static_cast<size_t>(C / 8), n = voxels * c8n;
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t v = i / c8n, c = (i % c8n) * 8;
-        __nv_bfloat16* d = dst + v * dst_ch + dst_off + c;
-        if (accumulate) {
-            Bf8 a = load8(src + v * src_ch + src_off + c);
-            const Bf8 b = load8(d);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) a.v[j] += b.v[j];
-            store8(d, a);
-        } else {
-            *reinterpret_cast<uint4*>(d) = *reinterpret_cast<const uint4*>(src + v * src_ch + src_off + c);
-        }
-    }
 }
 
 // g *= (act > 0): the gradient through a ReLU whose output is act; n is a
 // multiple of 8.
 __global__ void k_relu_backward(__nv_bfloat16* __restrict__ g, const __nv_bfloat16* __restrict__ act, size_t n) {
     for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n / 8; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const Bf8 a = load8(act + 8 * i);
         Bf8 v = load8(g + 8 * i);
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (!(a.v[j] > 0.0f)) v.v[j] = 0.0f;
+        relu_mask(v, load8(act + 8 * i));
         store8(g + 8 * i, v);
     }
 }
 
 // Mean squared error of the FP32 output against the target; writes the
 // gradient (channel 0 of a 16-channel BF16 tensor) and adds the loss sum.
-__global__ void k_mse(const float* __restrict__ out, const float* __restrict__ target, size_t n, __nv_bfloat16* __restrict__ grad16, double* __restrict__ loss_sum) {
+__global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, const float* __restrict__ target, size_t n, __nv_bfloat16* __restrict__ grad16, double* __restrict__ loss_sum) {
     double acc = 0.0;
     const float k = 2.0f / static_cast<float>(n);
     for (size_t v = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; v < n; v += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -210,9 +214,7 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
         reinterpret_cast<uint4*>(grad16 + v * 16)[0] = f;
         reinterpret_cast<uint4*>(grad16 + v * 16)[1] = z4;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss_sum, acc);
+    add_block_sum(acc, loss_sum);
 }
 
 // Adam on FP32 master weights; refreshes the BF16 copy and the transposed,

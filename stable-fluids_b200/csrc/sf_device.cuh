@@ -61,6 +61,12 @@ __device__ __forceinline__ size_t lin(int x, int y, int z, const Dims& d) {
     return static_cast<size_t>(x) + static_cast<size_t>(d.nx) * (static_cast<size_t>(y) + static_cast<size_t>(d.ny) * static_cast<size_t>(z));
 }
 
+// The same in 32 bits, for the gathers, whose instructions bound them: no grid
+// of 2^32 cells fits the memory of a device (the fields take 40 bytes a cell).
+__device__ __forceinline__ uint32_t lin32(int x, int y, int z, const Dims& d) {
+    return static_cast<uint32_t>(x) + static_cast<uint32_t>(d.nx) * (static_cast<uint32_t>(y) + static_cast<uint32_t>(d.ny) * static_cast<uint32_t>(z));
+}
+
 __device__ __forceinline__ int wrap_index(int c, int n) {
     c %= n;
     return c < 0 ? c + n : c;
@@ -261,12 +267,11 @@ __device__ __forceinline__ float3 sample_velocity3(const P* __restrict__ v, floa
     const Cell c = locate(x, y, z, h);
     float3 s[8];
     if (block_inside(c, d)) {
-        const size_t i = lin(c.x0, c.y0, c.z0, d);
-        const size_t sy = static_cast<size_t>(d.nx), sz = static_cast<size_t>(d.nx) * static_cast<size_t>(d.ny);
-        const size_t off[8] = {0, 1, sy, sy + 1, sz, sz + 1, sz + sy, sz + sy + 1};
+        const uint32_t i = lin32(c.x0, c.y0, c.z0, d), sy = static_cast<uint32_t>(d.nx), sz = sy * static_cast<uint32_t>(d.ny);
+        const P* const row[4] = {v + i, v + (i + sy), v + (i + sz), v + (i + sz + sy)};
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            const float4 q = ldg4(&v[i + off[k]]);
+            const float4 q = ldg4(row[k >> 1] + (k & 1));
             s[k] = make_float3(q.x, q.y, q.z);
         }
     } else {
@@ -292,7 +297,7 @@ __device__ __forceinline__ float3 trace_rk2(float x, float y, float z, int cx, i
     float3 v0;
     const Cell c = locate(x, y, z, h);
     if (c.tx == 0.0f && c.ty == 0.0f && c.tz == 0.0f && c.x0 == cx && c.y0 == cy && c.z0 == cz) {
-        const float4 q = ldg4(&v[lin(cx, cy, cz, d)]);
+        const float4 q = ldg4(v + lin32(cx, cy, cz, d));
         v0 = make_float3(q.x, q.y, q.z);
     } else {
         v0 = sample_velocity3(v, x, y, z, d, h, b);

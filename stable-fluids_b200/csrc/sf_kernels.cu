@@ -83,6 +83,12 @@ __global__ void k_force_pack(ForceArgs a) {
 // One RK2 trace per cell for all three components (the reference re-traces
 // per component, backend-cuda.cu:330-340; the trace is deterministic so the
 // results are identical), then a trilinear sample of the packed velocity.
+// The latency of the gathers and the instructions around them bound it (470 for
+// a scalar's cell, a quarter of them addresses before these were 32 bits): 256^3
+// in 298 us instead of 313, the scalar's in 356 instead of 405; in BF16 at
+// 384^3 the two gained 60 and 230 us (now 1350 and 1440). Five CTAs an SM: four and six take
+// 3 to 6 % longer for the velocity; without a bound the scalar's takes 64
+// registers, four CTAs, and 10 % longer.
 template <typename T, typename P>
 __device__ __forceinline__ void advect_velocity_block(uint3 blk, const P* __restrict__ v, T* __restrict__ ox, T* __restrict__ oy, T* __restrict__ oz, float dt, const Dims& d, float h, const FlowBC& b) {
     int x, y, z;
@@ -92,7 +98,7 @@ __device__ __forceinline__ void advect_velocity_block(uint3 blk, const P* __rest
     const float pz = __fmul_rn(static_cast<float>(z) + 0.5f, h);
     const float3 t = trace_rk2(px, py, pz, x, y, z, v, dt, d, h, b);
     const float3 s = sample_velocity3(v, t.x, t.y, t.z, d, h, b);
-    const size_t i = lin(x, y, z, d);
+    const uint32_t i = lin32(x, y, z, d);
     ox[i] = from_f<T>(s.x);
     oy[i] = from_f<T>(s.y);
     oz[i] = from_f<T>(s.z);
@@ -131,23 +137,20 @@ __device__ __forceinline__ void scalar_source_advect_block(uint3 blk, const P* _
     float s[8];
     if (block_inside(c, d)) {
         // the whole 2x2x2 block is inside: no ghost rule applies
-        const size_t i = lin(c.x0, c.y0, c.z0, d);
-        const size_t sy = static_cast<size_t>(d.nx), sz = static_cast<size_t>(d.nx) * static_cast<size_t>(d.ny);
+        const uint32_t i = lin32(c.x0, c.y0, c.z0, d), sy = static_cast<uint32_t>(d.nx), sz = sy * static_cast<uint32_t>(d.ny);
+        const uint32_t row[4] = {i, i + sy, i + sz, i + sz + sy};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const size_t j = i + static_cast<size_t>(k & 1) + ((k >> 1) & 1 ? sy : 0) + (k >> 2 ? sz : 0);
-            s[k] = __fmaf_rn(dt, __ldg(&src[j]), ldg_f(&q[j]));
-        }
+        for (int k = 0; k < 8; ++k) s[k] = __fmaf_rn(dt, __ldg(src + row[k >> 1] + (k & 1)), ldg_f(q + row[k >> 1] + (k & 1)));
     } else {
         const int bx = corner_base(c.x0, d.nx), by = corner_base(c.y0, d.ny), bz = corner_base(c.z0, d.nz);
 #pragma unroll
         for (int k = 0; k < 8; ++k) s[k] = sourced_scalar(q, src, dt, bx + (k & 1), by + ((k >> 1) & 1), bz + (k >> 2), d, sb);
     }
-    out[lin(x, y, z, d)] = from_f<T>(trilerp(s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], c));
+    out[lin32(x, y, z, d)] = from_f<T>(trilerp(s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], c));
 }
 
 template <typename T, typename P>
-__global__ void __launch_bounds__(256) k_scalar_source_advect(const P* __restrict__ v, const T* __restrict__ q, const float* __restrict__ src, T* __restrict__ out, float dt, Dims d, float h, FlowBC fb, ScalarBC sb) { scalar_source_advect_block<T, P>(blockIdx, v, q, src, out, dt, d, h, fb, sb); }
+__global__ void __launch_bounds__(256, 5) k_scalar_source_advect(const P* __restrict__ v, const T* __restrict__ q, const float* __restrict__ src, T* __restrict__ out, float dt, Dims d, float h, FlowBC fb, ScalarBC sb) { scalar_source_advect_block<T, P>(blockIdx, v, q, src, out, dt, d, h, fb, sb); }
 
 template <typename T>
 __global__ void k_scalar_source(T* __restrict__ q, const float* __restrict__ src, float dt, size_t n) {
@@ -461,7 +464,7 @@ __device__ __forceinline__ uint3 cell_block_of(uint32_t local, const Dims& d) {
     return batch_block(local, static_cast<uint32_t>((d.nx + kBX - 1) / kBX), static_cast<uint32_t>((d.ny + kBY - 1) / kBY));
 }
 
-__global__ void __launch_bounds__(256) k_batch_advect_velocity(BatchTable t) {
+__global__ void __launch_bounds__(256, 5) k_batch_advect_velocity(BatchTable t) {
     const uint32_t* first = t.first[SHAPE_CELL];
     for (uint32_t w = blockIdx.x; w < t.total[SHAPE_CELL]; w += gridDim.x) {
         const int si = batch_sim(first, t.nsims, w);
@@ -470,7 +473,7 @@ __global__ void __launch_bounds__(256) k_batch_advect_velocity(BatchTable t) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_batch_scalar_source_advect(BatchTable t) {
+__global__ void __launch_bounds__(256, 5) k_batch_scalar_source_advect(BatchTable t) {
     const uint32_t* first = t.first[SHAPE_CELL];
     for (uint32_t w = blockIdx.x; w < t.total[SHAPE_CELL]; w += gridDim.x) {
         const int si = batch_sim(first, t.nsims, w);

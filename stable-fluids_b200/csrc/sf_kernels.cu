@@ -86,9 +86,9 @@ __global__ void k_force_pack(ForceArgs a) {
 // The latency of the gathers and the instructions around them bound it (470 for
 // a scalar's cell, a quarter of them addresses before these were 32 bits): 256^3
 // in 298 us instead of 313, the scalar's in 356 instead of 405; in BF16 at
-// 384^3 the two gained 60 and 230 us (now 1350 and 1440). Five CTAs an SM: four and six take
-// 3 to 6 % longer for the velocity; without a bound the scalar's takes 64
-// registers, four CTAs, and 10 % longer.
+// 384^3 the two gained 60 and 230 us (now 1350 and 1440). Five CTAs an SM: four
+// and six take 3 to 6 % longer for the velocity; without a bound the scalar's
+// takes 64 registers, four CTAs, and 10 % longer.
 template <typename T, typename P>
 __device__ __forceinline__ void advect_velocity_block(uint3 blk, const P* __restrict__ v, T* __restrict__ ox, T* __restrict__ oy, T* __restrict__ oz, float dt, const Dims& d, float h, const FlowBC& b) {
     int x, y, z;

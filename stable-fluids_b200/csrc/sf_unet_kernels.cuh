@@ -133,9 +133,10 @@ __device__ __forceinline__ void relu_mask(Bf8& g, const Bf8& act) {
 
 // Gradient of an encoder level's output, which feeds the skip connection and
 // the pooling: channels [off, off + C) of the concatenation's gradient plus 1/8
-// of the coarse parent's, rounded to BF16, through the ReLU whose output is act (C
-// channels). Launch: row_grid(fine nx, C / 8, fine ny, fine nz). One pass over memory: a copy, an addition and a mask in
-// passes of their own took 86 us at 128^3 with 16 channels, this 48.
+// of the coarse parent's, rounded to BF16, through the ReLU whose output is act
+// (C channels). Launch: row_grid(fine nx, C / 8, fine ny, fine nz). Bound by
+// memory: a copy, an addition and a mask in passes of their own took 86 us at
+// 128^3 with 16 channels, this one pass 48.
 __global__ void k_skip_backward(const __nv_bfloat16* __restrict__ gcat, int cat_ch, int off, const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __restrict__ gcoarse, int C, Dims coarse, __nv_bfloat16* __restrict__ gfine) {
     const int c8n = C / 8, fnx = coarse.nx * 2, fny = coarse.ny * 2;
     const int i = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);

@@ -62,8 +62,9 @@ cudaError_t launch_stencil(const StencilArgs& a, cudaStream_t s);
 // only (the velocity components), in one launch where that is possible.
 cudaError_t launch_stencils(const StencilArgs* a, int n, cudaStream_t s);
 // The solves of a small grid held in the shared memory of a cluster
-// (sf_resident.cu); false (nothing launched) when they do not suit it.
-bool launch_resident(const StencilArgs* a, int n, cudaStream_t s, cudaError_t* e);
+// (sf_resident.cu); false (nothing launched) when they do not suit it or the
+// device refuses it.
+bool launch_resident(const StencilArgs* a, int n, cudaStream_t s);
 cudaError_t launch_divergence(float* div, const void* vx, const void* vy, const void* vz, Dims d, float h, const FlowBC& b, int bf16, cudaStream_t s);
 // u -= grad p (in place) and repack; with stats != nullptr also accumulates
 // the FP64 residual sums of the pressure system into stats.

@@ -48,6 +48,7 @@
 #include "sf_divide.cuh"
 #include "sf_f32x2.cuh"
 #include "sf_launch.h"
+#include "sf_per_device.h"
 #include "sf_stencil_tb.cuh"
 #include "sf_stencil_wave.cuh"
 
@@ -346,10 +347,11 @@ struct ResidentKernel {
 };
 
 // The kernel with its attributes set, and the cluster sizes the device takes
-// (looked up once: each query costs some 50 us of a context's creation).
+// (looked up once a device: each query costs some 50 us of a context's creation).
 template <bool PRESSURE, bool JACOBI, bool RAGGED, typename T>
 const ResidentKernel& resident_kernel() {
-    static const ResidentKernel r = [] {
+    static PerDevice<ResidentKernel> kernels;
+    return kernels.get([] {
         ResidentKernel k{k_resident<PRESSURE, JACOBI, RAGGED, T>, {}};
         if (cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentShared) != cudaSuccess || cudaFuncSetAttribute(k.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
@@ -363,8 +365,7 @@ const ResidentKernel& resident_kernel() {
         }
         cudaGetLastError();
         return k;
-    }();
-    return r;
+    });
 }
 
 template <bool RAGGED>
@@ -396,10 +397,10 @@ bool resident_shape(const Dims& d, int py, int pz, bool jacobi, ResidentArgs& a,
 
 // The solves of a[0 .. n - 1] (same grid, scheme, start, iterations and
 // coefficient; n <= 3) in one launch; false (nothing launched) when they do
-// not fit a cluster's shared memory or are asked for in another form.
-bool launch_resident(const StencilArgs* a, int n, cudaStream_t s, cudaError_t* e) {
+// not fit a cluster's shared memory or are asked for in another form, or when
+// the device refuses the launch.
+bool launch_resident(const StencilArgs* a, int n, cudaStream_t s) {
     const StencilArgs& f = a[0];
-    *e = cudaSuccess;
     if (n < 1 || n > kMaxSolves || f.per_pass != 0 || f.iterations < 1) return false;
     const size_t cells = static_cast<size_t>(f.dims.nx) * f.dims.ny * f.dims.nz;
     if (cells > (1u << 19)) return false;  // 16 CTAs hold at most 0.4 M cells
@@ -449,8 +450,11 @@ bool launch_resident(const StencilArgs* a, int n, cudaStream_t s, cudaError_t* e
     const int threads = static_cast<int>(std::min<long long>(kResidentThreads, std::max<long long>(128, (items + 31) / 32 * 32)));
     cudaLaunchAttribute attr{};
     const cudaLaunchConfig_t cfg = resident_config(n * best_size, best_size, threads, best_smem, s, attr);
-    *e = cudaLaunchKernelEx(&cfg, kern.kernel, static_cast<const ResidentArgs>(best));
-    if (*e == cudaSuccess && f.launches) *f.launches += 1;
+    if (cudaLaunchKernelEx(&cfg, kern.kernel, static_cast<const ResidentArgs>(best)) != cudaSuccess) {
+        cudaGetLastError();  // nothing was launched: the sweeps run instead
+        return false;
+    }
+    if (f.launches) *f.launches += 1;
     return true;
 }
 

@@ -1449,15 +1449,14 @@ bool launch_residual_sums_vec(const float* p, const float* div, Dims d, float h2
 }
 
 cudaError_t launch_stencils(const StencilArgs* a, int n, cudaStream_t s) {
+    if (launch_resident(a, n, s)) return cudaSuccess;
     cudaError_t e = cudaSuccess;
-    if (launch_resident(a, n, s, &e)) return e;
     for (int k = 0; k < n && e == cudaSuccess; ++k) e = launch_stencil(a[k], s);
     return e;
 }
 
 cudaError_t launch_stencil(const StencilArgs& a, cudaStream_t s) {
-    cudaError_t resident = cudaSuccess;
-    if (launch_resident(&a, 1, s, &resident)) return resident;
+    if (launch_resident(&a, 1, s)) return cudaSuccess;
     // per_pass: 0 (default) = one launch per Jacobi sweep, red-black solves
     // in the colour-split layout where the rows allow (one launch per
     // colour); 1 = one launch per sweep or per colour on the interleaved

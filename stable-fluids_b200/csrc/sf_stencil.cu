@@ -1058,7 +1058,7 @@ cudaError_t launch_wave_pass(const wave::WaveArgs& w, int sms, cudaStream_t s) {
     constexpr size_t smem = wave::WaveLayout<K, V, kWaveRows>::bytes;
     static_assert(smem <= 232448, "shared memory per CTA");
     auto kern = wave::k_wave<KIND, RB, K, V, kWaveRows>;
-    static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));  // the current device's
     if (attr != cudaSuccess) return attr;
     constexpr int ty = kWaveRows - 2 * K;
     const int tiles = (w.d.ny + ty - 1) / ty;
@@ -1192,7 +1192,7 @@ cudaError_t launch_tb_pass(const TbArgs& args, const CUtensorMap& mx, const CUte
     constexpr size_t smem = TbLayout<K, W, HH, ZP>::bytes;
     static_assert(smem <= 232448, "shared memory per CTA");
     auto kern = k_rbgs_tb<KIND, K, W, HH, ZP, NT>;
-    static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));  // the current device's
     if (attr != cudaSuccess) return attr;
     constexpr int HX = ((K + 3) / 4) * 4;
     const dim3 grid(static_cast<unsigned>((args.d.nx + W - 2 * HX - 1) / (W - 2 * HX)), static_cast<unsigned>((args.d.ny + HH - 2 * K - 1) / (HH - 2 * K)), static_cast<unsigned>((args.d.nz + z_chunk - 1) / z_chunk));

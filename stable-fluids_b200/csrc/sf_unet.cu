@@ -209,7 +209,7 @@ cudaError_t wgrad(const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw,
     CUtensorMap map_in{}, map_out{};
     if (!voxel_map(&map_in, in, CIN, d, wg::TX + 2, wg::TY + 2, C::TZ + 2) || !voxel_map(&map_out, dout, COUT, d, wg::TX, wg::TY, C::TZ)) return cudaErrorInvalidValue;
     const auto kern = wg::k_conv3d_wgrad<COUT>;
-    static const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES);
+    const cudaError_t attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::BYTES);  // the current device's
     if (attr != cudaSuccess) return attr;
     constexpr int groups = CIN / 16;
     const int tx = (d.nx + wg::TX - 1) / wg::TX, ty = (d.ny + wg::TY - 1) / wg::TY, tz = (d.nz + C::TZ - 1) / C::TZ;
@@ -237,7 +237,7 @@ struct ChainLaunch {
     }
     cudaError_t launch(Dims d, cudaStream_t s, unsigned* error) {
         if (!ok) return cudaErrorInvalidValue;
-        static const cudaError_t attr = cudaFuncSetAttribute(wg::k_conv3d_wgrad_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, wg::ChainCfg::BYTES);
+        const cudaError_t attr = cudaFuncSetAttribute(wg::k_conv3d_wgrad_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, wg::ChainCfg::BYTES);
         if (attr != cudaSuccess) return attr;
         const int voxels = d.nx * d.ny * d.nz;
         const int units = (voxels + wg::kSegmentUnit - 1) / wg::kSegmentUnit;

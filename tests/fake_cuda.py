@@ -4,9 +4,11 @@ nothing there; memory is host memory, and a tensor or array on the host serves
 where a device pointer is wanted."""
 
 import ctypes
+import functools
 import pathlib
 import shutil
 import subprocess
+import tempfile
 
 import pytest
 
@@ -15,19 +17,24 @@ PACKAGE = ROOT / "stable-fluids_b200"
 CUDA = pathlib.Path("/usr/local/cuda")
 
 
-def build(out):
+@functools.lru_cache(maxsize=None)
+def build():
     if not (shutil.which("nvcc") or (CUDA / "bin" / "nvcc").exists()):
         pytest.skip("no CUDA toolkit")
     subprocess.run(["make", "-s", "-j4", "-C", str(PACKAGE)], check=True, capture_output=True)
-    objects = sorted(str(p) for p in (PACKAGE / "_build").glob("*.o") if (PACKAGE / "csrc" / f"{p.stem}.cu").exists() or (PACKAGE / "csrc" / f"{p.stem}.cpp").exists())
-    so = out / "libstable-fluids-fake.so"
+    sources = [*(PACKAGE / "csrc").glob("*.cu"), *(PACKAGE / "csrc").glob("*.cpp")]
+    objects = [str(PACKAGE / "_build" / f"{p.stem}.o") for p in sorted(sources)]
+    folder = tempfile.TemporaryDirectory(prefix="fake-cuda-")
+    so = pathlib.Path(folder.name) / "libstable-fluids-fake.so"
     subprocess.run(["g++", "-std=c++20", "-O1", "-shared", "-fPIC", f"-I{CUDA / 'include'}", str(ROOT / "tests" / "fakes" / "cudart.cpp"), *objects, "-o", str(so), "-Wl,-Bsymbolic", "-Wl,--no-undefined", "-ldl"], check=True)
-    return so
+    return so, folder
 
 
 def load(sf, out):
-    """The library on the fake runtime; its fake_* functions are the tests' handles."""
-    lib = sf.load_library(build(out))
+    """The library on the fake runtime, as a process of its own would see it
+    (nothing looked up yet); its fake_* functions are the tests' handles."""
+    so, _ = build()
+    lib = sf.load_library(shutil.copy(so, out))
     lib.fake_set_device.argtypes = [ctypes.c_int]
     lib.fake_executed_of.argtypes = [ctypes.c_char_p]
     lib.fake_patch_copies.argtypes = [ctypes.c_size_t, ctypes.c_size_t, ctypes.c_uint]

@@ -3,14 +3,16 @@ GPU and then on another gets the same on both. The devices are those of a CUDA
 runtime without a GPU (fake_cuda.py), which refuses a launch that asks for more
 shared memory or a larger cluster than its device has allowed for the kernel."""
 
+import ctypes
+
 import pytest
 
 from tests import fake_cuda
 
 
-@pytest.fixture(scope="module")
-def fake(sf, tmp_path_factory):
-    return fake_cuda.load(sf, tmp_path_factory.mktemp("fake"))
+@pytest.fixture
+def fake(sf, tmp_path):
+    return fake_cuda.load(sf, tmp_path)
 
 
 def _step(sf, fake, n, scheme):
@@ -44,3 +46,33 @@ def test_a_refused_cluster_launch_takes_the_sweeps(sf, fake):
     assert _step(sf, fake, (40, 32, 24), sf.SCHEME_RBGS) > 11
     fake.fake_take_clusters(1)
     assert _step(sf, fake, (40, 32, 24), sf.SCHEME_RBGS) <= 11
+
+
+def test_gradients_on_a_second_device(sf, fake):
+    n = (16, 12, 8)
+    field = (ctypes.c_float * (n[0] * n[1] * n[2]))()
+    executed = []
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        net = ctypes.c_void_p()
+        assert fake.stable_fluids_b200_network_create(1, ctypes.byref(net)) == sf.RESULT_OK
+        before = fake.fake_executed()
+        assert fake.stable_fluids_b200_network_gradients(net, field, field, field, *n, 1.0, None, None, None) == sf.RESULT_OK
+        executed.append(fake.fake_executed() - before)
+        fake.stable_fluids_b200_network_destroy(net)
+    fake.fake_set_device(0)
+    assert fake.fake_refused() == 0
+    assert executed[0] == executed[1] > 0
+
+
+@pytest.mark.parametrize("n", [(128, 24, 16), (72, 24, 16)], ids=["wavefront passes", "TMA passes"])
+def test_blocked_passes_on_a_second_device(n, sf, fake):
+    o = sf.default_options(fake)
+    o.iterations_per_pass = 2
+    for device in (0, 1):
+        fake.fake_set_device(device)
+        rc, ctx = fake_cuda.create(sf, fake, n, o)
+        assert rc == sf.RESULT_OK
+        fake.stable_fluids_destroy_context_cuda(ctx)
+    fake.fake_set_device(0)
+    assert fake.fake_refused() == 0

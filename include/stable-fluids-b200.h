@@ -91,7 +91,10 @@ STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_default_options(StableFl
  * null for the defaults; environment overrides are NOT applied here). */
 STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_create_context(const StableFluidsContextCreateDesc* desc, const StableFluidsB200Options* options, void** out_context, StableFluidsScalarFieldHandle* out_scalar_field_handles, uint32_t out_scalar_field_handle_capacity, StableFluidsVectorFieldHandle* out_vector_field_handles, uint32_t out_vector_field_handle_capacity);
 
-/* Waits for the context stream and returns the statistics of the last step. */
+/* Waits for the context stream and returns the statistics of the last step.
+ * BACKEND_FAILURE also when a kernel of this or an earlier step gave up one of
+ * its bounded waits: its solve was not finished and the fields are not those
+ * of a step, so the context reports it from then on. */
 STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_get_step_stats(void* context, StableFluidsB200StepStats* out_stats);
 
 /* Staged update of a vector field, for callers that upload a new field from

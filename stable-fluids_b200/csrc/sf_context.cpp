@@ -875,6 +875,7 @@ StableFluidsResult stable_fluids_b200_get_step_stats(void* context, StableFluids
     if (cudaMemcpyAsync(c.host_stats, c.stats, sizeof(sfb::DeviceStats), cudaMemcpyDeviceToHost, c.stream) != cudaSuccess) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
     if (cudaStreamSynchronize(c.stream) != cudaSuccess) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
     const auto& d = *c.host_stats;
+    if (d.error != 0) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;  // a kernel's bounded wait gave up: the fields are not a step's
     StableFluidsB200StepStats o{};
     o.rel_residual = c.residual_enabled ? d.rel_residual : -1.0;
     o.rhs_norm = c.residual_enabled ? d.rhs_norm : 0.0;

@@ -178,6 +178,10 @@ STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_get_step_info(void* cont
  *
  * A network object serves one stream at a time (its activation buffers are
  * shared by every call); all entry points except predict are synchronous.
+ * When a kernel gives up one of its bounded waits, gradients and train_step
+ * return BACKEND_FAILURE and leave the parameters as they were (after predict
+ * on a grid: the next of them on that grid; in a step:
+ * stable_fluids_b200_get_step_stats).
  */
 STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_network_create(uint32_t seed, void** out_network);
 STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_network_destroy(void* network);

@@ -362,9 +362,9 @@ struct Stages {
             const float h2c = (2.0f * h()) * (2.0f * h());
             ok(launch_restrict2(c.divergence, c.coarse_b, c.dims, c.stream));
             ok(launch_restrict2(c.pressure, c.coarse_p, c.dims, c.stream));
-            if (ok(net::predict(c.network, c.coarse_b, h2c, c.coarse_p, c.coarse_out, c.coarse_dims(), c.stream, &predicted, &c), 0)) launches += predicted;
+            if (ok(net::predict(c.network, c.coarse_b, h2c, c.coarse_p, c.coarse_out, c.coarse_dims(), c.stream, &predicted, &c, &c.stats->error), 0)) launches += predicted;
             ok(launch_prolong_add(c.coarse_out, c.coarse_p, c.pressure, c.dims, c.stream));
-        } else if (ok(net::predict(c.network, c.divergence, h() * h(), c.pressure, c.pressure, c.dims, c.stream, &predicted, &c), 0)) {
+        } else if (ok(net::predict(c.network, c.divergence, h() * h(), c.pressure, c.pressure, c.dims, c.stream, &predicted, &c, &c.stats->error), 0)) {
             launches += predicted;
         }
         if (trial > 0) {

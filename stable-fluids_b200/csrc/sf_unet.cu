@@ -70,8 +70,11 @@ struct Buffers {
     float* target = nullptr;  // FP32 scaled training target
     // gradients (BF16)
     __nv_bfloat16 *g16 = nullptr, *gd0b = nullptr, *gd0a = nullptr, *gcat0 = nullptr, *gd1b = nullptr, *gd1a = nullptr, *gcat1 = nullptr, *gbb = nullptr, *gba = nullptr, *gp1 = nullptr, *ge1b = nullptr, *ge1a = nullptr, *gp0 = nullptr, *ge0b = nullptr, *ge0a = nullptr;
-    double* sums = nullptr;  // [0] sum of squares of b, [1] loss sum
+    double* sums = nullptr;  // [0] sum of squares of b, [1] loss sum, [2] the error word
     float* scale = nullptr;
+
+    // set by a kernel whose bounded wait gave up (results are then invalid)
+    unsigned* error() const { return reinterpret_cast<unsigned*>(sums + 2); }
 
     Buffers() = default;
     Buffers(const Buffers&) = delete;
@@ -90,7 +93,6 @@ struct Net {
     float* v = nullptr;
     __nv_bfloat16* w16 = nullptr;   // BF16 weights [tap][cout][cin] per layer
     __nv_bfloat16* w16t = nullptr;  // BF16 transposed, tap-flipped weights [tap][cin][cout] (data gradient)
-    unsigned* error = nullptr;      // set by a convolution whose bounded wait gave up
     int adam_t = 0;
     // Buffer sets by grid size and owner, kept until the network is
     // destroyed (or the owner releases them) so that step graphs holding
@@ -111,7 +113,6 @@ struct Net {
         cudaFree(v);
         cudaFree(w16);
         cudaFree(w16t);
-        cudaFree(error);
     }
 };
 
@@ -293,7 +294,6 @@ Net* create_net(uint32_t seed) {
     const size_t fb = off * sizeof(float);
     if (cudaMalloc(&n->w, fb) != cudaSuccess || cudaMalloc(&n->g, fb) != cudaSuccess || cudaMalloc(&n->m, fb) != cudaSuccess || cudaMalloc(&n->v, fb) != cudaSuccess) return nullptr;
     if (cudaMalloc(&n->w16, off * sizeof(__nv_bfloat16)) != cudaSuccess || cudaMalloc(&n->w16t, off * sizeof(__nv_bfloat16)) != cudaSuccess) return nullptr;
-    if (cudaMalloc(&n->error, sizeof(unsigned)) != cudaSuccess || cudaMemset(n->error, 0, sizeof(unsigned)) != cudaSuccess) return nullptr;
     // He initialisation over the real fan-in (the output layer 10x smaller);
     // padded input channels and padded output channels of the last layer are
     // zero; biases zero.
@@ -370,7 +370,7 @@ cudaError_t ensure_buffers(Net* n, Dims d, const void* owner = nullptr) {
     items.push_back({reinterpret_cast<void**>(&b->target), b->n0 * sizeof(float)});
     }
     items.push_back({reinterpret_cast<void**>(&b->out), b->n0 * sizeof(float)});
-    items.push_back({reinterpret_cast<void**>(&b->sums), 2 * sizeof(double)});
+    items.push_back({reinterpret_cast<void**>(&b->sums), 3 * sizeof(double)});
     items.push_back({reinterpret_cast<void**>(&b->scale), sizeof(float)});
     size_t total = 0;
     for (const auto& it : items) total += (it.bytes + 255) & ~static_cast<size_t>(255);
@@ -406,7 +406,7 @@ float* GB(Net* n, int l) { return n->g + n->layers[l].off + n->layers[l].wn; }
 
 // Forward pass from b (scaled inside) and p_prev; leaves the FP32 output in
 // buf->out and every activation in place for the backward pass. 18 kernels.
-cudaError_t forward(Net* n, const float* b, float b_factor, const float* p_prev, cudaStream_t s) {
+cudaError_t forward(Net* n, const float* b, float b_factor, const float* p_prev, unsigned* error, cudaStream_t s) {
     Buffers& B = *n->buf;
     cudaError_t e;
     SFB_TRY(cudaMemsetAsync(B.sums, 0, sizeof(double), s));
@@ -414,21 +414,21 @@ cudaError_t forward(Net* n, const float* b, float b_factor, const float* p_prev,
     k_finish_scale<<<1, 32, 0, s>>>(B.sums, static_cast<double>(B.n0), B.scale);
     k_pack_input<<<blocks_for(B.n0), 256, 0, s>>>(b, p_prev, B.scale, b_factor, B.in, B.n0);
     SFB_TRY(cudaGetLastError());
-    SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.in, W(n, E0A), Bias(n, E0A), B.e0a, 16, 0, B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.e0a, W(n, E0B), Bias(n, E0B), B.e0b, 16, 0, B.d0, s, n->error));
+    SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.in, W(n, E0A), Bias(n, E0A), B.e0a, 16, 0, B.d0, s, error));
+    SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.e0a, W(n, E0B), Bias(n, E0B), B.e0b, 16, 0, B.d0, s, error));
     k_pool2<<<row_grid(B.d1.nx, 2, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.e0b, 16, 0, B.p0, 16, B.d1);
-    SFB_TRY(conv_any(16, 32, tc::RELU_BF16, B.p0, W(n, E1A), Bias(n, E1A), B.e1a, 32, 0, B.d1, s, n->error));
-    SFB_TRY(conv_any(32, 32, tc::RELU_BF16, B.e1a, W(n, E1B), Bias(n, E1B), B.e1b, 32, 0, B.d1, s, n->error));
+    SFB_TRY(conv_any(16, 32, tc::RELU_BF16, B.p0, W(n, E1A), Bias(n, E1A), B.e1a, 32, 0, B.d1, s, error));
+    SFB_TRY(conv_any(32, 32, tc::RELU_BF16, B.e1a, W(n, E1B), Bias(n, E1B), B.e1b, 32, 0, B.d1, s, error));
     k_pool2<<<row_grid(B.d2.nx, 4, B.d2.ny, B.d2.nz), 256, 0, s>>>(B.e1b, 32, 0, B.p1, 32, B.d2);
-    SFB_TRY(conv_any(32, 64, tc::RELU_BF16, B.p1, W(n, BA), Bias(n, BA), B.ba, 64, 0, B.d2, s, n->error));
-    SFB_TRY(conv_any(64, 64, tc::RELU_BF16, B.ba, W(n, BB), Bias(n, BB), B.bb, 64, 0, B.d2, s, n->error));
+    SFB_TRY(conv_any(32, 64, tc::RELU_BF16, B.p1, W(n, BA), Bias(n, BA), B.ba, 64, 0, B.d2, s, error));
+    SFB_TRY(conv_any(64, 64, tc::RELU_BF16, B.ba, W(n, BB), Bias(n, BB), B.bb, 64, 0, B.d2, s, error));
     k_upsample2_concat<<<row_grid(B.d1.nx, 12, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.bb, 64, B.d2, B.e1b, 32, B.cat1);
-    SFB_TRY(conv_any(96, 32, tc::RELU_BF16, B.cat1, W(n, D1A), Bias(n, D1A), B.d1a, 32, 0, B.d1, s, n->error));
-    SFB_TRY(conv_any(32, 32, tc::RELU_BF16, B.d1a, W(n, D1B), Bias(n, D1B), B.d1b, 32, 0, B.d1, s, n->error));
+    SFB_TRY(conv_any(96, 32, tc::RELU_BF16, B.cat1, W(n, D1A), Bias(n, D1A), B.d1a, 32, 0, B.d1, s, error));
+    SFB_TRY(conv_any(32, 32, tc::RELU_BF16, B.d1a, W(n, D1B), Bias(n, D1B), B.d1b, 32, 0, B.d1, s, error));
     k_upsample2_concat<<<row_grid(B.d0.nx, 6, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.d1b, 32, B.d1, B.e0b, 16, B.cat0);
-    SFB_TRY(conv_any(48, 16, tc::RELU_BF16, B.cat0, W(n, D0A), Bias(n, D0A), B.d0a, 16, 0, B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.d0a, W(n, D0B), Bias(n, D0B), B.d0b, 16, 0, B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 16, tc::LINEAR_F32_CH0, B.d0b, W(n, OUT), Bias(n, OUT), B.out, 1, 0, B.d0, s, n->error));
+    SFB_TRY(conv_any(48, 16, tc::RELU_BF16, B.cat0, W(n, D0A), Bias(n, D0A), B.d0a, 16, 0, B.d0, s, error));
+    SFB_TRY(conv_any(16, 16, tc::RELU_BF16, B.d0a, W(n, D0B), Bias(n, D0B), B.d0b, 16, 0, B.d0, s, error));
+    SFB_TRY(conv_any(16, 16, tc::LINEAR_F32_CH0, B.d0b, W(n, OUT), Bias(n, OUT), B.out, 1, 0, B.d0, s, error));
     return cudaGetLastError();
 }
 
@@ -444,47 +444,47 @@ cudaError_t backward(Net* n, cudaStream_t s) {
     ChainLaunch chain;
     // out layer (linear)
     if (chained) chain.add(B.d0b, 16, B.g16, GW(n, OUT), GB(n, OUT), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.d0b, B.g16, GW(n, OUT), GB(n, OUT), B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.g16, WT(n, OUT), nullptr, B.gd0b, 16, 0, B.d0, s, n->error));
+    else SFB_TRY(wgrad_any(16, 16, B.d0b, B.g16, GW(n, OUT), GB(n, OUT), B.d0, s, B.error()));
+    SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.g16, WT(n, OUT), nullptr, B.gd0b, 16, 0, B.d0, s, B.error()));
     // d0b, d0a (input of d0a: cat0 = [up(d1b) | e0b])
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.gd0b, B.d0b, B.n0 * 16);
     if (chained) chain.add(B.d0a, 16, B.gd0b, GW(n, D0B), GB(n, D0B), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.d0a, B.gd0b, GW(n, D0B), GB(n, D0B), B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.gd0b, WT(n, D0B), nullptr, B.gd0a, 16, 0, B.d0, s, n->error));
+    else SFB_TRY(wgrad_any(16, 16, B.d0a, B.gd0b, GW(n, D0B), GB(n, D0B), B.d0, s, B.error()));
+    SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.gd0b, WT(n, D0B), nullptr, B.gd0a, 16, 0, B.d0, s, B.error()));
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.gd0a, B.d0a, B.n0 * 16);
     if (chained) chain.add(B.cat0, 48, B.gd0a, GW(n, D0A), GB(n, D0A), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(48, 16, B.cat0, B.gd0a, GW(n, D0A), GB(n, D0A), B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 48, tc::LINEAR_BF16, B.gd0a, WT(n, D0A), nullptr, B.gcat0, 48, 0, B.d0, s, n->error));
+    else SFB_TRY(wgrad_any(48, 16, B.cat0, B.gd0a, GW(n, D0A), GB(n, D0A), B.d0, s, B.error()));
+    SFB_TRY(conv_any(16, 48, tc::LINEAR_BF16, B.gd0a, WT(n, D0A), nullptr, B.gcat0, 48, 0, B.d0, s, B.error()));
     k_upsample2_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat0, 48, 0, 32, B.d1, B.d1b, B.gd1b);
     // d1b, d1a (input of d1a: cat1 = [up(bb) | e1b])
-    SFB_TRY(wgrad_any(32, 32, B.d1a, B.gd1b, GW(n, D1B), GB(n, D1B), B.d1, s, n->error));
-    SFB_TRY(conv_any(32, 32, tc::LINEAR_BF16, B.gd1b, WT(n, D1B), nullptr, B.gd1a, 32, 0, B.d1, s, n->error));
+    SFB_TRY(wgrad_any(32, 32, B.d1a, B.gd1b, GW(n, D1B), GB(n, D1B), B.d1, s, B.error()));
+    SFB_TRY(conv_any(32, 32, tc::LINEAR_BF16, B.gd1b, WT(n, D1B), nullptr, B.gd1a, 32, 0, B.d1, s, B.error()));
     k_relu_backward<<<blocks_for(B.n1 * 32 / 8), 256, 0, s>>>(B.gd1a, B.d1a, B.n1 * 32);
-    SFB_TRY(wgrad_any(96, 32, B.cat1, B.gd1a, GW(n, D1A), GB(n, D1A), B.d1, s, n->error));
-    SFB_TRY(conv_any(32, 96, tc::LINEAR_BF16, B.gd1a, WT(n, D1A), nullptr, B.gcat1, 96, 0, B.d1, s, n->error));
+    SFB_TRY(wgrad_any(96, 32, B.cat1, B.gd1a, GW(n, D1A), GB(n, D1A), B.d1, s, B.error()));
+    SFB_TRY(conv_any(32, 96, tc::LINEAR_BF16, B.gd1a, WT(n, D1A), nullptr, B.gcat1, 96, 0, B.d1, s, B.error()));
     k_upsample2_backward<<<row_grid(B.d2.nx, 8, B.d2.ny, B.d2.nz), 256, 0, s>>>(B.gcat1, 96, 0, 64, B.d2, B.bb, B.gbb);
     // bottleneck
-    SFB_TRY(wgrad_any(64, 64, B.ba, B.gbb, GW(n, BB), GB(n, BB), B.d2, s, n->error));
-    SFB_TRY(conv_any(64, 64, tc::LINEAR_BF16, B.gbb, WT(n, BB), nullptr, B.gba, 64, 0, B.d2, s, n->error));
+    SFB_TRY(wgrad_any(64, 64, B.ba, B.gbb, GW(n, BB), GB(n, BB), B.d2, s, B.error()));
+    SFB_TRY(conv_any(64, 64, tc::LINEAR_BF16, B.gbb, WT(n, BB), nullptr, B.gba, 64, 0, B.d2, s, B.error()));
     k_relu_backward<<<blocks_for(B.n2 * 64 / 8), 256, 0, s>>>(B.gba, B.ba, B.n2 * 64);
-    SFB_TRY(wgrad_any(32, 64, B.p1, B.gba, GW(n, BA), GB(n, BA), B.d2, s, n->error));
-    SFB_TRY(conv_any(64, 32, tc::LINEAR_BF16, B.gba, WT(n, BA), nullptr, B.gp1, 32, 0, B.d2, s, n->error));
+    SFB_TRY(wgrad_any(32, 64, B.p1, B.gba, GW(n, BA), GB(n, BA), B.d2, s, B.error()));
+    SFB_TRY(conv_any(64, 32, tc::LINEAR_BF16, B.gba, WT(n, BA), nullptr, B.gp1, 32, 0, B.d2, s, B.error()));
     // e1b receives the skip (channels 64..95 of cat1) and the pooled path
     k_skip_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat1, 96, 64, B.e1b, B.gp1, 32, B.d2, B.ge1b);
-    SFB_TRY(wgrad_any(32, 32, B.e1a, B.ge1b, GW(n, E1B), GB(n, E1B), B.d1, s, n->error));
-    SFB_TRY(conv_any(32, 32, tc::LINEAR_BF16, B.ge1b, WT(n, E1B), nullptr, B.ge1a, 32, 0, B.d1, s, n->error));
+    SFB_TRY(wgrad_any(32, 32, B.e1a, B.ge1b, GW(n, E1B), GB(n, E1B), B.d1, s, B.error()));
+    SFB_TRY(conv_any(32, 32, tc::LINEAR_BF16, B.ge1b, WT(n, E1B), nullptr, B.ge1a, 32, 0, B.d1, s, B.error()));
     k_relu_backward<<<blocks_for(B.n1 * 32 / 8), 256, 0, s>>>(B.ge1a, B.e1a, B.n1 * 32);
-    SFB_TRY(wgrad_any(16, 32, B.p0, B.ge1a, GW(n, E1A), GB(n, E1A), B.d1, s, n->error));
-    SFB_TRY(conv_any(32, 16, tc::LINEAR_BF16, B.ge1a, WT(n, E1A), nullptr, B.gp0, 16, 0, B.d1, s, n->error));
+    SFB_TRY(wgrad_any(16, 32, B.p0, B.ge1a, GW(n, E1A), GB(n, E1A), B.d1, s, B.error()));
+    SFB_TRY(conv_any(32, 16, tc::LINEAR_BF16, B.ge1a, WT(n, E1A), nullptr, B.gp0, 16, 0, B.d1, s, B.error()));
     // e0b: skip (channels 32..47 of cat0) + pooled path
     k_skip_backward<<<row_grid(B.d0.nx, 2, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.gcat0, 48, 32, B.e0b, B.gp0, 16, B.d1, B.ge0b);
     if (chained) chain.add(B.e0a, 16, B.ge0b, GW(n, E0B), GB(n, E0B), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.e0a, B.ge0b, GW(n, E0B), GB(n, E0B), B.d0, s, n->error));
-    SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.ge0b, WT(n, E0B), nullptr, B.ge0a, 16, 0, B.d0, s, n->error));
+    else SFB_TRY(wgrad_any(16, 16, B.e0a, B.ge0b, GW(n, E0B), GB(n, E0B), B.d0, s, B.error()));
+    SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.ge0b, WT(n, E0B), nullptr, B.ge0a, 16, 0, B.d0, s, B.error()));
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.ge0a, B.e0a, B.n0 * 16);
     if (chained) chain.add(B.in, 16, B.ge0a, GW(n, E0A), GB(n, E0A), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.in, B.ge0a, GW(n, E0A), GB(n, E0A), B.d0, s, n->error));
-    if (chained) SFB_TRY(chain.launch(B.d0, s, n->error));
+    else SFB_TRY(wgrad_any(16, 16, B.in, B.ge0a, GW(n, E0A), GB(n, E0A), B.d0, s, B.error()));
+    if (chained) SFB_TRY(chain.launch(B.d0, s, B.error()));
     return cudaGetLastError();
 }
 
@@ -496,16 +496,24 @@ __global__ void k_make_target(const float* __restrict__ pt, const float* __restr
 
 cudaError_t loss_and_gradients(Net* n, const float* b, float b_factor, const float* p_prev, const float* p_target, double* loss, cudaStream_t s) {
     cudaError_t e;
-    SFB_TRY(forward(n, b, b_factor, p_prev, s));
     Buffers& B = *n->buf;
+    SFB_TRY(forward(n, b, b_factor, p_prev, B.error(), s));
     k_make_target<<<blocks_for(B.n0), 256, 0, s>>>(p_target, p_prev, B.scale, B.target, B.n0);
     SFB_TRY(cudaMemsetAsync(B.sums + 1, 0, sizeof(double), s));
     k_mse<<<sum_blocks(B.n0), 256, 0, s>>>(B.out, B.target, B.n0, B.g16, B.sums + 1);
     SFB_TRY(backward(n, s));
-    double sum = 0.0;
-    SFB_TRY(cudaMemcpyAsync(&sum, B.sums + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
+    struct {
+        double loss;
+        unsigned error, pad;
+    } sums{};
+    static_assert(sizeof(sums) == 2 * sizeof(double));
+    SFB_TRY(cudaMemcpyAsync(&sums, B.sums + 1, sizeof(sums), cudaMemcpyDeviceToHost, s));
     SFB_TRY(cudaStreamSynchronize(s));
-    if (loss) *loss = sum / static_cast<double>(B.n0);
+    if (sums.error != 0) {
+        SFB_TRY(cudaMemsetAsync(B.error(), 0, sizeof(unsigned), s));
+        return cudaErrorLaunchTimeout;
+    }
+    if (loss) *loss = sums.loss / static_cast<double>(B.n0);
     return cudaSuccess;
 }
 
@@ -540,10 +548,10 @@ void release(Net* n, const void* owner) {
     }
 }
 
-cudaError_t predict(Net* n, const float* b, float b_factor, const float* p_prev, float* p0, Dims d, cudaStream_t s, int* launches, const void* owner) {
+cudaError_t predict(Net* n, const float* b, float b_factor, const float* p_prev, float* p0, Dims d, cudaStream_t s, int* launches, const void* owner, unsigned* error) {
     cudaError_t e = ensure_buffers(n, d, owner);
     if (e != cudaSuccess) return e;
-    if ((e = forward(n, b, b_factor, p_prev, s)) != cudaSuccess) return e;
+    if ((e = forward(n, b, b_factor, p_prev, error != nullptr ? error : n->buf->error(), s)) != cudaSuccess) return e;
     k_unpack_output<<<blocks_for(n->buf->n0), 256, 0, s>>>(n->buf->out, p_prev, n->buf->scale, p0, n->buf->n0);
     if (launches) *launches += kPredictKernels;
     return cudaGetLastError();
@@ -614,7 +622,7 @@ StableFluidsResult stable_fluids_b200_network_set_parameters(void* network, cons
 StableFluidsResult stable_fluids_b200_network_predict(void* network, const float* divergence, const float* previous_pressure, int32_t nx, int32_t ny, int32_t nz, float cell_size, float* out_pressure, void* stream) {
     if (network == nullptr || divergence == nullptr || out_pressure == nullptr) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
     const sfb::Dims d{nx, ny, nz, 0};
-    return status(sfb::net::predict(static_cast<Net*>(network), divergence, cell_size * cell_size, previous_pressure, out_pressure, d, static_cast<cudaStream_t>(stream), nullptr, nullptr));
+    return status(sfb::net::predict(static_cast<Net*>(network), divergence, cell_size * cell_size, previous_pressure, out_pressure, d, static_cast<cudaStream_t>(stream), nullptr, nullptr, nullptr));
 }
 
 StableFluidsResult stable_fluids_b200_network_gradients(void* network, const float* divergence, const float* previous_pressure, const float* target_pressure, int32_t nx, int32_t ny, int32_t nz, float cell_size, double* out_loss, float* out_host_gradients, void* stream) {

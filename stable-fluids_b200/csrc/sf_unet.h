@@ -30,7 +30,9 @@ void release(Net* n, const void* owner);
 
 // p0 = p_prev + net(b_factor * b, p_prev) / scale on stream s, with the
 // buffers of (d, owner); p_prev may be null (zero) and may alias p0. Adds
-// kPredictKernels to *launches.
-cudaError_t predict(Net* n, const float* b, float b_factor, const float* p_prev, float* p0, Dims d, cudaStream_t s, int* launches, const void* owner);
+// kPredictKernels to *launches. A kernel whose bounded wait gives up sets
+// *error (null: a word of the network's, which the next gradients on this grid
+// report).
+cudaError_t predict(Net* n, const float* b, float b_factor, const float* p_prev, float* p0, Dims d, cudaStream_t s, int* launches, const void* owner, unsigned* error);
 
 }  // namespace sfb::net

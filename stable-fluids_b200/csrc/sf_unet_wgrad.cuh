@@ -164,7 +164,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
             }
         }
         __syncthreads();  // the stage is free
-        if (tid == 0 && k + 2 < mine) load(k + 2);
+        if (tid == 0 && k + 2 < mine && !*abort) load(k + 2);
+    }
+    if (*abort) {  // a wait gave up: nothing is added, and copies still under way land before the CTA leaves
+        __nanosleep(1000000);
+        return;
     }
     // the shares' sums into the first share's registers, through shared memory
     if constexpr (SPLIT > 1) {
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(kChainThreads) k_conv3d_wgrad_chain(const __gr
         const unsigned char* const stage = smem + i % kChainStages * C::STAGE;
         const uint32_t st = base + static_cast<uint32_t>(i % kChainStages * C::STAGE);
         if (helps) {
-            if (i + 1 < n) load(i + 1);  // into the stage of chunk i - 1
+            if (i + 1 < n && !*abort) load(i + 1);  // into the stage of chunk i - 1
         } else if (warp < 3) {
             // the tap (dz, dy, warp - 1): one chain of MMAs per accumulator,
             // each block's operands fetched before the MMAs of the one before
@@ -356,6 +360,10 @@ __global__ void __launch_bounds__(kChainThreads) k_conv3d_wgrad_chain(const __gr
             }
         }
         __syncthreads();
+    }
+    if (*abort) {  // as in k_conv3d_wgrad
+        __nanosleep(1000000);
+        return;
     }
     if (warp < 3) {
         const int tap = static_cast<int>(blockIdx.y) * 3 + warp, co = lane >> 2, ci = g.c0 + 2 * (lane & 3);

@@ -12,7 +12,7 @@ namespace sfb::net {
 struct Net;
 
 // Kernels one predict() enqueues.
-constexpr int kPredictKernels = 21;
+constexpr int kPredictKernels = 19;
 
 // Sets the FP32 master parameters from host memory (synchronous) and
 // refreshes the BF16 copies; resets the optimizer state.

@@ -48,7 +48,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <climits>
 
 #include "sf_device.cuh"
 #include "sf_divide.cuh"
@@ -154,13 +153,13 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     // Each thread owns one float4 of every step-th row of the block.
     const int tid = static_cast<int>(threadIdx.x), nt = static_cast<int>(blockDim.x);
     const int rows = ny * nz, step = nt / a.lanes;
-    const int k0 = 4 * (tid % a.lanes), first = tid / a.lanes < step ? tid / a.lanes : INT_MAX / 2;
+    const int edges = 2 * (ny + nz);  // the rows on the block's edges
+    const int k0 = 4 * (tid % a.lanes), first = tid / a.lanes < step ? tid / a.lanes : rows + edges;  // beyond both: no row
     int* const row_at = reinterpret_cast<int*>(rhs + 2 * rhs_colour);  // 2 x the row's offset in an array, + 1 where its red cells sit at odd x
     // The rows on the block's edges, {row, target, face, mbarrier}: a pad row
     // beside it is a ghost row of the other colour's array here (its offset;
     // mbarrier 0) or the neighbour's row of the same colour (its address in the
     // cluster, for the array at offset 0, and the neighbour's mbarrier).
-    const int edges = 2 * (ny + nz);
     int4* const edge_at = reinterpret_cast<int4*>(row_at + (a.rows_y * a.rows_z + 3) / 4 * 4);
     const uint32_t bar_addr = static_cast<uint32_t>(__cvta_generic_to_shared(bar));
 

@@ -18,6 +18,7 @@
 #include "sf_batch.cuh"
 #include "sf_device.cuh"
 #include "sf_divide.cuh"
+#include "sf_half_offsets.h"
 #include "sf_launch.h"
 #include "sf_stencil_tb.cuh"
 #include "sf_stencil_wave.cuh"
@@ -575,14 +576,12 @@ __device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, co
     const bool px = g.periodic[0] != 0, py = g.periodic[1] != 0, pz = g.periodic[2] != 0;
     const divide::Divisor div = divide::make_divisor(KIND == KIND_PRESSURE ? 6.0f : 1.0f + 6.0f * coef);
     const float k = KIND == KIND_PRESSURE ? -coef : coef;
-    const int hsz = hx * d.ny * B;  // bytes of a half plane
-    // rows y - 1, y + 1 (offsets in the half plane) and their face ghosts
+    const HalfOffsets off = half_offsets<B>(d, y, k0, px, py, pz);
+    // face ghosts of rows y - 1, y + 1
     const bool gy_lo = !py && y == 0, gy_hi = !py && y == d.ny - 1, y_face = gy_lo || gy_hi;
-    const int oy_lo = B * (y > 0 ? -hx : (py ? (d.ny - 1) * hx : 0)), oy_hi = B * (y + 1 < d.ny ? hx : (py ? -(d.ny - 1) * hx : 0));
     // the extra x neighbour: k0 - 1 (rows whose u cells sit at even x) or
     // k0 + 4 (odd x), wrapped or replaced by a ghost at a face
     const bool gx_lo = !px && k0 == 0, gx_hi = !px && k0 + 4 == hx;
-    const int ox_lo = B * (k0 > 0 ? -1 : (px ? hx - 1 : 0)), ox_hi = B * (k0 + 4 < hx ? 4 : (px ? 4 - hx : 3));
     const float gk_lo = g.k[XM], gk_hi = g.k[XP];
     const int gm_lo = g.mode[XM], gm_hi = g.mode[XP];
     // One plane: `near` the plane on the side the march comes from, `cur`; loads
@@ -590,10 +589,10 @@ __device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, co
     // thread (cell 0 on rows whose cells sit at even x, cell 3 on odd ones)
     // takes its x ghost, from its own value in u; y faces (the whole row) and z
     // faces (the whole plane) sit behind a branch interior threads skip.
-    const auto plane = [&](uint32_t i, bool odd, bool z_lo, bool z_hi, float4 near, float4 cur, int far) {
+    const auto plane = [&](uint32_t i, bool odd, bool z_lo, bool z_hi, float4 near, float4 cur, uint32_t far) {
         const float4 next = ld4v(at_byte(v, i + far));
-        float ext = ld1v(at_byte(v, i + (odd ? ox_hi : ox_lo)));
-        float4 c = ld4v(at_byte(v, i + oy_lo)), e = ld4v(at_byte(v, i + oy_hi));
+        float ext = ld1v(at_byte(v, i + (odd ? off.x_hi : off.x_lo)));
+        float4 c = ld4v(at_byte(v, i + off.y_lo)), e = ld4v(at_byte(v, i + off.y_hi));
         const float4 r = ld4v(at_byte(w, i));
         const bool gx = odd ? gx_hi : gx_lo;
         float self_x = 0.0f;
@@ -637,16 +636,16 @@ __device__ __forceinline__ void rb_half_block(uint32_t bx, uint32_t bz, T* u, co
     };
     const uint32_t row = static_cast<uint32_t>(B) * static_cast<uint32_t>(k0 + hx * y);
     // DOWN marches the chunk from its top plane (see jacobi_vec4_block)
-    const int z_first = DOWN ? ze - 1 : zb, step = DOWN ? -hsz : hsz;
-    const int wrap = pz ? (d.nz - 1) * hsz : 0;  // from the bottom plane to the top one (itself on a face)
-    uint32_t i = row + static_cast<uint32_t>(z_first) * static_cast<uint32_t>(hsz);
+    const int z_first = DOWN ? ze - 1 : zb;
+    const uint32_t up = off.plane, down = 0u - off.plane, step = DOWN ? down : up;
+    uint32_t i = row + static_cast<uint32_t>(z_first) * off.plane;
     float4 cur = ld4v(at_byte(v, i));
-    float4 near = ld4v(at_byte(v, i + (DOWN ? (ze < d.nz ? hsz : -wrap) : (zb > 0 ? -hsz : wrap))));
+    float4 near = ld4v(at_byte(v, i + (DOWN ? (ze < d.nz ? up : 0u - off.wrap) : (zb > 0 ? down : off.wrap))));
     bool odd = ((y + z_first + colour) & 1) != 0;
 #pragma unroll 1
     for (int z = z_first; DOWN ? z >= zb : z < ze; z += DOWN ? -1 : 1, i += step, odd = !odd) {
         const bool bottom = z == 0, top = z == d.nz - 1;
-        const float4 next = plane(i, odd, !pz && bottom, !pz && top, near, cur, DOWN ? (bottom ? wrap : -hsz) : (top ? -wrap : hsz));
+        const float4 next = plane(i, odd, !pz && bottom, !pz && top, near, cur, DOWN ? (bottom ? off.wrap : down) : (top ? 0u - off.wrap : up));
         near = cur;
         cur = next;
     }

@@ -255,7 +255,7 @@ struct ChainLaunch {
 cudaError_t wgrad_any(int cin, int cout, const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw, float* db, Dims d, cudaStream_t s, unsigned* error) {
 #define SFB_WG(CI, CO) \
     if (cin == CI && cout == CO) return wgrad<CI, CO>(in, dout, dw, db, d, s, error);
-    SFB_WG(16, 16) SFB_WG(16, 32) SFB_WG(32, 32) SFB_WG(32, 64) SFB_WG(64, 64) SFB_WG(96, 32) SFB_WG(48, 16)
+    SFB_WG(16, 32) SFB_WG(32, 32) SFB_WG(32, 64) SFB_WG(64, 64) SFB_WG(96, 32)
 #undef SFB_WG
     return cudaErrorInvalidValue;
 }
@@ -314,8 +314,13 @@ Net* create_net(uint32_t seed) {
     return n.release();
 }
 
+// The kernels count voxels in 32 bits: no device holds the buffers of so many
+// (325 bytes a voxel for a prediction, 700 with the gradients).
+constexpr size_t kMaxVoxels = (1ull << 31) - 4096;
+
 cudaError_t ensure_buffers(Net* n, Dims d, const void* owner = nullptr) {
     if (d.nx % 4 || d.ny % 4 || d.nz % 4 || d.nx < 4 || d.ny < 4 || d.nz < 4) return cudaErrorInvalidValue;
+    if (static_cast<size_t>(d.nx) * d.ny >= kMaxVoxels || static_cast<size_t>(d.nx) * d.ny * d.nz >= kMaxVoxels) return cudaErrorMemoryAllocation;
     for (auto& set : n->sets)
         if (set->owner == owner && set->d0.nx == d.nx && set->d0.ny == d.ny && set->d0.nz == d.nz) {
             n->buf = set.get();
@@ -440,20 +445,16 @@ cudaError_t backward(Net* n, cudaStream_t s) {
     Buffers& B = *n->buf;
     cudaError_t e;
     SFB_TRY(cudaMemsetAsync(n->g, 0, n->nparams * sizeof(float), s));
-    const bool chained = B.n0 < (1ull << 31) - 4096;  // the chain kernel counts voxels in 32 bits
     ChainLaunch chain;
     // out layer (linear)
-    if (chained) chain.add(B.d0b, 16, B.g16, GW(n, OUT), GB(n, OUT), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.d0b, B.g16, GW(n, OUT), GB(n, OUT), B.d0, s, B.error()));
+    chain.add(B.d0b, 16, B.g16, GW(n, OUT), GB(n, OUT), static_cast<long long>(B.n0));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.g16, WT(n, OUT), nullptr, B.gd0b, 16, 0, B.d0, s, B.error()));
     // d0b, d0a (input of d0a: cat0 = [up(d1b) | e0b])
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.gd0b, B.d0b, B.n0 * 16);
-    if (chained) chain.add(B.d0a, 16, B.gd0b, GW(n, D0B), GB(n, D0B), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.d0a, B.gd0b, GW(n, D0B), GB(n, D0B), B.d0, s, B.error()));
+    chain.add(B.d0a, 16, B.gd0b, GW(n, D0B), GB(n, D0B), static_cast<long long>(B.n0));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.gd0b, WT(n, D0B), nullptr, B.gd0a, 16, 0, B.d0, s, B.error()));
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.gd0a, B.d0a, B.n0 * 16);
-    if (chained) chain.add(B.cat0, 48, B.gd0a, GW(n, D0A), GB(n, D0A), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(48, 16, B.cat0, B.gd0a, GW(n, D0A), GB(n, D0A), B.d0, s, B.error()));
+    chain.add(B.cat0, 48, B.gd0a, GW(n, D0A), GB(n, D0A), static_cast<long long>(B.n0));
     SFB_TRY(conv_any(16, 48, tc::LINEAR_BF16, B.gd0a, WT(n, D0A), nullptr, B.gcat0, 48, 0, B.d0, s, B.error()));
     k_upsample2_backward<<<row_grid(B.d1.nx, 4, B.d1.ny, B.d1.nz), 256, 0, s>>>(B.gcat0, 48, 0, 32, B.d1, B.d1b, B.gd1b);
     // d1b, d1a (input of d1a: cat1 = [up(bb) | e1b])
@@ -478,13 +479,11 @@ cudaError_t backward(Net* n, cudaStream_t s) {
     SFB_TRY(conv_any(32, 16, tc::LINEAR_BF16, B.ge1a, WT(n, E1A), nullptr, B.gp0, 16, 0, B.d1, s, B.error()));
     // e0b: skip (channels 32..47 of cat0) + pooled path
     k_skip_backward<<<row_grid(B.d0.nx, 2, B.d0.ny, B.d0.nz), 256, 0, s>>>(B.gcat0, 48, 32, B.e0b, B.gp0, 16, B.d1, B.ge0b);
-    if (chained) chain.add(B.e0a, 16, B.ge0b, GW(n, E0B), GB(n, E0B), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.e0a, B.ge0b, GW(n, E0B), GB(n, E0B), B.d0, s, B.error()));
+    chain.add(B.e0a, 16, B.ge0b, GW(n, E0B), GB(n, E0B), static_cast<long long>(B.n0));
     SFB_TRY(conv_any(16, 16, tc::LINEAR_BF16, B.ge0b, WT(n, E0B), nullptr, B.ge0a, 16, 0, B.d0, s, B.error()));
     k_relu_backward<<<blocks_for(B.n0 * 16 / 8), 256, 0, s>>>(B.ge0a, B.e0a, B.n0 * 16);
-    if (chained) chain.add(B.in, 16, B.ge0a, GW(n, E0A), GB(n, E0A), static_cast<long long>(B.n0));
-    else SFB_TRY(wgrad_any(16, 16, B.in, B.ge0a, GW(n, E0A), GB(n, E0A), B.d0, s, B.error()));
-    if (chained) SFB_TRY(chain.launch(B.d0, s, B.error()));
+    chain.add(B.in, 16, B.ge0a, GW(n, E0A), GB(n, E0A), static_cast<long long>(B.n0));
+    SFB_TRY(chain.launch(B.d0, s, B.error()));
     return cudaGetLastError();
 }
 

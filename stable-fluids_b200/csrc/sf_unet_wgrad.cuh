@@ -63,13 +63,13 @@ template <int COUT>
 struct Cfg {
     static constexpr int MT = COUT / 16;                 // tiles of 16 output channels
     static constexpr int SPLIT = 4 / MT;                 // shares of a tile's voxels
-    static constexpr int TZ = COUT == 16 ? 4 : 2;
+    static constexpr int TZ = 2;
     static constexpr int IN_CHUNK = (TX + 2) * (TY + 2) * (TZ + 2) * 16;
     static constexpr int OUT_CHUNK = TX * TY * TZ * 16;
     static constexpr int STAGE = 2 * IN_CHUNK + COUT / 8 * OUT_CHUNK;
     static constexpr int BAR_OFF = 2 * STAGE;            // full[2], abort flag
     static constexpr int BYTES = BAR_OFF + 32;
-    static_assert(COUT == 16 || COUT == 32 || COUT == 64, "output channels");
+    static_assert(COUT == 32 || COUT == 64, "output channels");
     static_assert(IN_CHUNK % 128 == 0 && OUT_CHUNK % 128 == 0 && BYTES <= 232448, "shared memory");
     static_assert(SPLIT == 1 || 3 * MT * (SPLIT - 1) * 32 * 76 * 4 <= 2 * STAGE, "the reduction over the shares reuses the stages");
 };

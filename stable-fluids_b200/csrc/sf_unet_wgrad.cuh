@@ -336,12 +336,24 @@ __global__ void __launch_bounds__(kChainThreads) k_conv3d_wgrad_chain(const __gr
                 ldmatrix4_trans(st + lane_a + static_cast<uint32_t>(k * 512), fa[k & 1]);
                 ldmatrix4_trans(flags[k >> 2] & (1u << (8 * (k & 3))) ? st + lane_b + static_cast<uint32_t>(k * 512) : zero, fb[k & 1]);
             };
-            fetch(0);
+            const int blocks = (v_end - v_first - i * kChunk + 15) / 16;  // of this segment; past it lies another's dout
+            if (blocks >= kChunk / 16) {
+                fetch(0);
 #pragma unroll
-            for (int k = 0; k < kChunk / 16; ++k) {
-                if (k + 1 < kChunk / 16) fetch(k + 1);
-                mma_16816(acc[0], fa[k & 1], fb[k & 1][0], fb[k & 1][1]);
-                mma_16816(acc[1], fa[k & 1], fb[k & 1][2], fb[k & 1][3]);
+                for (int k = 0; k < kChunk / 16; ++k) {
+                    if (k + 1 < kChunk / 16) fetch(k + 1);
+                    mma_16816(acc[0], fa[k & 1], fb[k & 1][0], fb[k & 1][1]);
+                    mma_16816(acc[1], fa[k & 1], fb[k & 1][2], fb[k & 1][3]);
+                }
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < blocks; ++k) {
+                    const unsigned flag = stage[C::FLAGS + voxel * (kChunk / 16) + k];
+                    ldmatrix4_trans(st + lane_a + static_cast<uint32_t>(k * 512), fa[0]);
+                    ldmatrix4_trans((flag >> warp) & 1u ? st + lane_b + static_cast<uint32_t>(k * 512) : zero, fb[0]);
+                    mma_16816(acc[0], fa[0], fb[0][0], fb[0][1]);
+                    mma_16816(acc[1], fa[0], fb[0][2], fb[0][3]);
+                }
             }
         } else if (bias) {
             // FP32 sums of dout, 8 channels of every 16th voxel a lane

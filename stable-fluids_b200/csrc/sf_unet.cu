@@ -214,7 +214,7 @@ cudaError_t wgrad(const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw,
     if (attr != cudaSuccess) return attr;
     constexpr int groups = CIN / 16;
     const int tx = (d.nx + wg::TX - 1) / wg::TX, ty = (d.ny + wg::TY - 1) / wg::TY, tz = (d.nz + C::TZ - 1) / C::TZ;
-    const wg::Args a{dw, db, CIN, tx, ty, tx * ty * tz, error};
+    const wg::Args a{dw, db, CIN, tx, ty, tx * ty * tz, d, error};
     const int per_group = std::max(1, std::min(a.tiles, sm_count() / groups));
     kern<<<dim3(static_cast<unsigned>(per_group), groups), wg::kThreads, C::BYTES, s>>>(map_in, map_out, a);
     return cudaGetLastError();

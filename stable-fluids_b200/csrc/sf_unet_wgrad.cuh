@@ -6,8 +6,9 @@
 // A CTA owns 16 input channels and walks tiles of TX x TY x TZ voxels. The TMA
 // brings a tile's dout and the halo of `in` into shared memory as 8-channel
 // chunks of 16-byte rows, one row a voxel (out-of-grid voxels as zeros: the
-// convolution's padding, and tiles that reach past the grid add nothing), two
-// tiles in flight. Per tap the tile is a GEMM with M = 16 output channels,
+// convolution's padding), two tiles in flight. What a tile has past the grid is
+// left out, or meets zeros on both sides where a block of 16 reaches past it:
+// dout's zeros alone would make NaN of an infinity in the halo. Per tap the tile is a GEMM with M = 16 output channels,
 // N = 16 input channels and K = its voxels, 16 consecutive x at a time; the
 // tap's shift is an offset of whole rows. Both operands lie K-major in rows of
 // channels, which is what ldmatrix.trans turns into mma.sync fragments.
@@ -67,7 +68,8 @@ struct Cfg {
     static constexpr int IN_CHUNK = (TX + 2) * (TY + 2) * (TZ + 2) * 16;
     static constexpr int OUT_CHUNK = TX * TY * TZ * 16;
     static constexpr int STAGE = 2 * IN_CHUNK + COUT / 8 * OUT_CHUNK;
-    static constexpr int BAR_OFF = 2 * STAGE;            // full[2], abort flag
+    static constexpr int ZERO = 2 * STAGE;               // rows of zeros, as far as the taps of one row reach
+    static constexpr int BAR_OFF = ZERO + (2 * (TX + 2) + 2 + 1) * 16;  // full[2], abort flag
     static constexpr int BYTES = BAR_OFF + 32;
     static_assert(COUT == 32 || COUT == 64, "output channels");
     static_assert(IN_CHUNK % 128 == 0 && OUT_CHUNK % 128 == 0 && BYTES <= 232448, "shared memory");
@@ -79,6 +81,7 @@ struct Args {
     float* db;      // COUT
     int cin;        // input channels of the layer (16 a CTA: blockIdx.y)
     int tiles_x, tiles_y, tiles;
+    Dims d;
     unsigned* error;
 };
 
@@ -108,12 +111,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    for (int i = tid; i < (C::BAR_OFF - C::ZERO) / 16; i += kThreads) *reinterpret_cast<uint4*>(smem + C::ZERO + 16 * i) = make_uint4(0, 0, 0, 0);
     __syncthreads();
     const int c0 = 16 * static_cast<int>(blockIdx.y);
     const int mine = a.tiles > static_cast<int>(blockIdx.x) ? (a.tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1 : 0;
-    const auto load = [&](int k) {  // tile k of this CTA into stage k & 1 (one thread)
+    const auto corner = [&](int k) {  // of tile k of this CTA
         const int tile = static_cast<int>(blockIdx.x) + k * static_cast<int>(gridDim.x);
-        const int x = tile % a.tiles_x * TX, y = tile / a.tiles_x % a.tiles_y * TY, z = tile / (a.tiles_x * a.tiles_y) * TZ;
+        return make_int3(tile % a.tiles_x * TX, tile / a.tiles_x % a.tiles_y * TY, tile / (a.tiles_x * a.tiles_y) * TZ);
+    };
+    const auto load = [&](int k) {  // tile k into stage k & 1 (one thread)
+        const auto [x, y, z] = corner(k);
         const uint32_t st = base + static_cast<uint32_t>((k & 1) * C::STAGE), bar = full(k & 1);
         tc::mbar_expect_tx(bar, static_cast<uint32_t>(C::STAGE));
         for (int c = 0; c < 2; ++c) tc::tma_load_4d(st + static_cast<uint32_t>(c * C::IN_CHUNK), &map_in, c0 + 8 * c, x - 1, y - 1, z - 1, bar);
@@ -138,26 +145,32 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
     // (dout) the matrices are (chunk 0, k 0-7), (chunk 1, k 0-7), (chunk 0,
     // k 8-15), (chunk 1, k 8-15); for B (in) chunk and k change places
     const uint32_t lane_a = static_cast<uint32_t>(((lane >> 3) & 1) * C::OUT_CHUNK + (((lane >> 4) & 1) * 8 + (lane & 7)) * 16);
-    const uint32_t lane_b = static_cast<uint32_t>(((lane >> 4) & 1) * C::IN_CHUNK + (((lane >> 3) & 1) * 8 + (lane & 7)) * 16);
+    const int voxel = ((lane >> 3) & 1) * 8 + (lane & 7);  // of a block of 16: the row whose address this lane gives for B
+    const uint32_t lane_b = static_cast<uint32_t>(((lane >> 4) & 1) * C::IN_CHUNK + voxel * 16);
     for (int k = 0; k < mine; ++k) {
-        const bool ok = tc::mbar_wait(full(k & 1), static_cast<uint32_t>((k >> 1) & 1), abort, a.error);
+        const bool ok = __all_sync(0xffffffffu, tc::mbar_wait(full(k & 1), static_cast<uint32_t>((k >> 1) & 1), abort, a.error));
         const uint32_t st = base + static_cast<uint32_t>((k & 1) * C::STAGE);
         const uint32_t out = st + static_cast<uint32_t>(2 * C::IN_CHUNK + 2 * mt * C::OUT_CHUNK) + lane_a;
         const uint32_t in = st + static_cast<uint32_t>(dz * PY * PX * 16) + lane_b;
+        const int3 at = corner(k);
+        const int x_end = a.d.nx - at.x, y_end = a.d.ny - at.y, z_end = a.d.nz - at.z;  // of the grid, seen from the tile
         // rows (z, y) of the tile, this warp's share of them
 #pragma unroll 1
         for (int r = share * (TY * TZ / SPLIT); ok && r < (share + 1) * (TY * TZ / SPLIT); ++r) {
+            if (r % TY >= y_end || r / TY >= z_end) continue;
             const uint32_t row_out = out + static_cast<uint32_t>(r * TX * 16);
             const uint32_t row_in = in + static_cast<uint32_t>((r / TY * PY + r % TY) * PX * 16);
 #pragma unroll
             for (int h = 0; h < TX / 16; ++h) {
+                if (16 * h >= x_end) break;
+                const uint32_t in_h = 16 * h + voxel < x_end ? row_in + static_cast<uint32_t>(h * 256) : base + static_cast<uint32_t>(C::ZERO);
                 uint32_t fa[4];
                 ldmatrix4_trans(row_out + static_cast<uint32_t>(h * 256), fa);
                 if (bias) mma_16816(sum, fa, 0x3F803F80u, 0x3F803F80u);  // times ones
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
                     uint32_t fb[4];
-                    ldmatrix4_trans(row_in + static_cast<uint32_t>((t / 3 * PX + t % 3 + h * 16) * 16), fb);
+                    ldmatrix4_trans(in_h + static_cast<uint32_t>((t / 3 * PX + t % 3) * 16), fb);
                     mma_16816(acc[t][0], fa, fb[0], fb[1]);
                     mma_16816(acc[t][1], fa, fb[2], fb[3]);
                 }

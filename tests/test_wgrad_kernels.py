@@ -42,3 +42,10 @@ def test_an_infinity_beside_a_segment(check):
     """16 channels: an infinity in the gradient is in the sums it belongs to and in
     no other; the zeros that stand for what is outside a segment must not meet it."""
     assert _differing(check("inf"), ("->16",)) == []
+
+
+@pytest.mark.gpu
+def test_an_infinity_at_the_last_column(check):
+    """32 and 64 channels: an infinity among the activations beside voxels that a
+    tile has past the grid, and in the gradient."""
+    assert _differing(check("inf"), ("->32", "->64")) == []

@@ -73,7 +73,7 @@ struct Cfg {
     static constexpr int BYTES = BAR_OFF + 32;
     static_assert(COUT == 32 || COUT == 64, "output channels");
     static_assert(IN_CHUNK % 128 == 0 && OUT_CHUNK % 128 == 0 && BYTES <= 232448, "shared memory");
-    static_assert(SPLIT == 1 || 3 * MT * (SPLIT - 1) * 32 * 76 * 4 <= 2 * STAGE, "the reduction over the shares reuses the stages");
+    static_assert(SPLIT == 1 || 3 * MT * (SPLIT - 1) * 32 * 74 * 4 <= 2 * STAGE, "the reduction over the shares reuses the stages");
 };
 
 struct Args {
@@ -132,15 +132,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
     }
     const int dz = warp % 3, mt = warp / 3 % C::MT, share = warp / (3 * C::MT);
     const bool bias = dz == 1 && blockIdx.y == 0;  // these warps sum dout itself, too
-    float acc[9][2][4], sum[4];
+    float acc[9][2][4], sum[2];  // sum: of dout, rows lane / 4 and lane / 4 + 8 of the tile's 16 channels
 #pragma unroll
     for (int t = 0; t < 9; ++t)
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int i = 0; i < 4; ++i) acc[t][n][i] = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) sum[i] = 0.0f;
+    sum[0] = sum[1] = 0.0f;
     // lane l gives ldmatrix the address of row l % 8 of matrix l / 8: for A
     // (dout) the matrices are (chunk 0, k 0-7), (chunk 1, k 0-7), (chunk 0,
     // k 8-15), (chunk 1, k 8-15); for B (in) chunk and k change places
@@ -166,7 +165,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
                 const uint32_t in_h = 16 * h + voxel < x_end ? row_in + static_cast<uint32_t>(h * 256) : base + static_cast<uint32_t>(C::ZERO);
                 uint32_t fa[4];
                 ldmatrix4_trans(row_out + static_cast<uint32_t>(h * 256), fa);
-                if (bias) mma_16816(sum, fa, 0x3F803F80u, 0x3F803F80u);  // times ones
+                if (bias) {  // FP32 sums: the tensor cores would round theirs towards zero
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[i & 1] += __uint_as_float(fa[i] << 16) + __uint_as_float(fa[i] & 0xffff0000u);
+                }
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
                     uint32_t fb[4];
@@ -188,28 +190,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
         float* const part = reinterpret_cast<float*>(smem);
         __syncthreads();
         if (share > 0) {
-            float* const p = part + (((share - 1) * 3 * C::MT + mt * 3 + dz) * 76) * 32 + lane;
+            float* const p = part + (((share - 1) * 3 * C::MT + mt * 3 + dz) * 74) * 32 + lane;
 #pragma unroll
             for (int t = 0; t < 9; ++t)
 #pragma unroll
                 for (int n = 0; n < 2; ++n)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) p[(t * 8 + n * 4 + i) * 32] = acc[t][n][i];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) p[(72 + i) * 32] = sum[i];
+            p[72 * 32] = sum[0];
+            p[73 * 32] = sum[1];
         }
         __syncthreads();
         if (share > 0) return;
         for (int s = 0; s < SPLIT - 1; ++s) {
-            const float* const p = part + ((s * 3 * C::MT + mt * 3 + dz) * 76) * 32 + lane;
+            const float* const p = part + ((s * 3 * C::MT + mt * 3 + dz) * 74) * 32 + lane;
 #pragma unroll
             for (int t = 0; t < 9; ++t)
 #pragma unroll
                 for (int n = 0; n < 2; ++n)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) acc[t][n][i] += p[(t * 8 + n * 4 + i) * 32];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) sum[i] += p[(72 + i) * 32];
+            sum[0] += p[72 * 32];
+            sum[1] += p[73 * 32];
         }
     }
     if (mine == 0) return;
@@ -224,9 +226,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3d_wgrad(const __grid_const
             atomicAdd(w + 8 * a.cin, acc[t][n][2]);
             atomicAdd(w + 8 * a.cin + 1, acc[t][n][3]);
         }
-    if (bias && (lane & 3) == 0) {
-        atomicAdd(a.db + co, sum[0]);
-        atomicAdd(a.db + co + 8, sum[2]);
+    if (bias) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {  // over the four lanes of a row
+            sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 1);
+            sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 2);
+            if ((lane & 3) == 0) atomicAdd(a.db + co + 8 * i, sum[i]);
+        }
     }
 }
 

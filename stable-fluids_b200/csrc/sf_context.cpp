@@ -543,6 +543,10 @@ StableFluidsResult create(const StableFluidsContextCreateDesc* desc, const Stabl
     if (env) apply_env_overrides(options);
     if (!validate_options(options)) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
 
+    // The kernels index cells in 32 bits (lin32). The fields take 48 to 60 bytes
+    // a cell, 206 GB or more for 2^32 of them.
+    if (static_cast<uint64_t>(cfg.nx) * static_cast<uint64_t>(cfg.ny) > kMaxCells / static_cast<uint64_t>(cfg.nz)) return STABLE_FLUIDS_RESULT_OUT_OF_MEMORY;
+
     std::unique_ptr<Context> c{new (std::nothrow) Context{}};
     if (!c) return STABLE_FLUIDS_RESULT_OUT_OF_MEMORY;
     c->config = cfg;

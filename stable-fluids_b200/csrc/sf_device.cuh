@@ -61,8 +61,8 @@ __device__ __forceinline__ size_t lin(int x, int y, int z, const Dims& d) {
     return static_cast<size_t>(x) + static_cast<size_t>(d.nx) * (static_cast<size_t>(y) + static_cast<size_t>(d.ny) * static_cast<size_t>(z));
 }
 
-// The same in 32 bits, for the gathers, whose instructions bound them: no grid
-// of 2^32 cells fits the memory of a device (the fields take 40 bytes a cell).
+// The same in 32 bits, for the gathers, whose instructions bound them: a grid
+// has fewer than 2^32 cells (kMaxCells, checked when a context is created).
 __device__ __forceinline__ uint32_t lin32(int x, int y, int z, const Dims& d) {
     return static_cast<uint32_t>(x) + static_cast<uint32_t>(d.nx) * (static_cast<uint32_t>(y) + static_cast<uint32_t>(d.ny) * static_cast<uint32_t>(z));
 }

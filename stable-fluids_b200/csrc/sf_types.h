@@ -16,6 +16,9 @@ struct Dims {
     int32_t pad = 0;
 };
 
+// Most cells of a grid (create refuses more): a cell's index has 32 bits.
+constexpr uint64_t kMaxCells = 0xffffffffull;
+
 // Flow boundary, flattened from StableFluidsFlowBoundaryConfig.
 struct FlowBC {
     int32_t type[6];      // StableFluidsFlowBoundaryType per face

@@ -762,6 +762,8 @@ def reference_arm(sf, args, scene, world, rank, local):
     needs = read_calibration(args, args.warmup, args.steps)
     if needs is None:
         return {"impl": "reference", "unavailable": f"bench_calibration.json does not cover steps {args.warmup}..{args.warmup + args.steps - 1} of the {n}^3 scene at tolerance {args.tolerance:g}; run `python bench.py --calibrate --calibrate-steps {args.warmup + args.steps}`"}
+    if not orc.REF_LIB_PATH.exists():
+        return {"impl": "reference", "unavailable": "the reference backend is not built (oracle/_ref; oracle/Makefile builds it where its sources are)"}
     lib = sf.load_library(orc.REF_LIB_PATH)
     mean_need = int(round(statistics.mean(needs)))
     with Clocks(local, not args.no_clocks) as clk:

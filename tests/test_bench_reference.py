@@ -1,18 +1,17 @@
 """The benchmark's reference arm without a reference library: one line that says
-so, and a clean exit."""
+so."""
 
-import json
-import pathlib
-import subprocess
+import importlib
 import sys
 
-ROOT = pathlib.Path(__file__).resolve().parent.parent
+from oracle import oracle
 
 
-def test_missing_reference_is_one_line():
-    code = "import pathlib, sys; from oracle import oracle; oracle.REF_LIB_PATH = pathlib.Path('/nowhere/lib.so'); sys.argv = ['bench.py', '--impl', 'reference', '--steps', '20', '--warmup', '5']; import bench; bench.main()"
-    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
-    assert r.returncode == 0, r.stderr
-    line = json.loads(r.stdout.splitlines()[-1])
-    assert line["impl"] == "reference" and set(line) == {"impl", "unavailable"}
+def test_missing_reference_is_one_line(sf, monkeypatch, tmp_path):
+    bench = importlib.import_module("bench")
+    monkeypatch.setattr(oracle, "REF_LIB_PATH", tmp_path / "lib.so")
+    monkeypatch.setattr(sys, "argv", ["bench.py", "--impl", "reference", "--steps", "20", "--warmup", "5"])
+    args = bench.parse()
+    line = bench.reference_arm(sf, args, sf.scenes.config1(n=args.size), 1, 0, 0)
+    assert set(line) == {"impl", "unavailable"} and line["impl"] == "reference"
     assert "\n" not in line["unavailable"]

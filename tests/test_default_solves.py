@@ -115,3 +115,52 @@ def test_resident_solves_match_sweeps(n, walls, form, sf, lib, cuda):
     # the resident form ran: three launches for the five solves
     assert sweep_kernels - kernels >= 4 * DIFFUSE + PRESSURE - 3
     _assert_same(resident, sweeps)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("start", ["previous", "tolerance", "learned"])
+@pytest.mark.parametrize("scheme", ["SCHEME_RBGS", "SCHEME_JACOBI"])
+@pytest.mark.parametrize("n,walls", [((24, 20, 16), "stam"), ((28, 36, 20), "mixed"), ((20, 12, 8), "periodic"), ((34, 17, 12), "periodic_z"), ((31, 18, 14), "periodic_y")],
+                         ids=lambda v: v if isinstance(v, str) else "x".join(map(str, v)))
+def test_resident_solves_from_other_starts(n, walls, scheme, start, sf, lib, cuda):
+    """The pressure from the previous step's, in the intervals of a solve to a
+    tolerance, and on both candidates of a learned start."""
+    if start == "learned" and any(k % 4 for k in n):
+        pytest.skip("the network takes grids of multiples of four")
+    if walls == "periodic_z":
+        sc = sf.scenes
+        flow = [sf.FLOW_NO_SLIP_WALL, sf.FLOW_OUTFLOW, sf.FLOW_FREE_SLIP_WALL, sf.FLOW_NO_SLIP_WALL, sf.FLOW_PERIODIC, sf.FLOW_PERIODIC]
+        scalar = [sf.SCALAR_FIXED_VALUE, sf.SCALAR_ZERO_FLUX, sf.SCALAR_ZERO_FLUX, sf.SCALAR_FIXED_VALUE, sf.SCALAR_PERIODIC, sf.SCALAR_PERIODIC]
+        scene = _scene(sf, n, "stam")
+        scene = sf.scenes.plume("default", n, diffuse_iterations=DIFFUSE, pressure_iterations=PRESSURE, sources=scene.meta["sources"], velocity_seed=3, steps=3,
+                                walls=(sc.flow_boundary(flow, [(0, 0.03, -0.01)] + [(0, 0, 0)] * 5, [0, 0.25, 0, 0, 0, 0]), sc.scalar_boundary(scalar, [0.25, 0, 0, 0.5, 0, 0])))
+    else:
+        scene = _scene(sf, n, walls)
+    got = []
+    for per_pass in (0, 1):
+        o = sf.default_options(lib)
+        o.scheme, o.iterations_per_pass, o.compute_residual = getattr(sf, scheme), per_pass, 1
+        o.warm_start = sf.WARM_START_LEARNED if start == "learned" else sf.WARM_START_PREVIOUS
+        o.warm_start_trial_iterations = 3
+        if start == "tolerance":
+            o.residual_tolerance, o.residual_check_interval, o.max_pressure_iterations = 1e-4, 6, 60
+        sim = sf.Simulation(scene.config, scene.scalars, scene.vectors, lib=lib, options=o)
+        if start == "learned":
+            with sf.WarmStartNetwork(seed=3, lib=lib) as net:
+                net.attach(sim)
+                sf.scenes.run(sim, scene)
+                out = C.collect_outputs(sim, sf, C.Case(scene.name, scene.config, scene.scalars, scene.vectors, scene.steps))
+                stats = sim.stats()
+                sf.WarmStartNetwork.detach(sim)
+        else:
+            sf.scenes.run(sim, scene)
+            out = C.collect_outputs(sim, sf, C.Case(scene.name, scene.config, scene.scalars, scene.vectors, scene.steps))
+            stats = sim.stats()
+        got.append((out, stats, sim.info().kernels_per_step))
+        sim.close()
+    (a, sa, ka), (b, sb, kb) = got
+    _assert_same(a, b)
+    assert (sa.pressure_iterations, sa.hit_cap, sa.used_fallback) == (sb.pressure_iterations, sb.hit_cap, sb.used_fallback)
+    # FP64 sums of squares of at most 20160 cells, in the order of their atomics
+    assert abs(sa.rel_residual - sb.rel_residual) <= 20160 * 2.0**-53 * sb.rel_residual
+    assert ka < kb

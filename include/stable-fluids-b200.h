@@ -53,7 +53,9 @@ typedef enum StableFluidsB200Storage {
 typedef struct StableFluidsB200Options {
     uint32_t scheme;                  /* StableFluidsB200Scheme */
     uint32_t warm_start;              /* StableFluidsB200WarmStart */
-    int32_t iterations_per_pass;      /* 0 = automatic (single sweeps; red-black solves in the
+    int32_t iterations_per_pass;      /* 0 = automatic (a whole solve in one launch where the grid
+                                       * fits the shared memory of a thread block cluster, at most
+                                       * 2^19 cells; else single sweeps, red-black solves in the
                                        * colour-split layout where rows are a multiple of 8 cells);
                                        * 1 = one launch per sweep / colour on the interleaved field;
                                        * >= 2 = temporally blocked passes of that many iterations */

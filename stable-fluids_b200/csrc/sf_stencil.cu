@@ -1456,9 +1456,10 @@ cudaError_t launch_stencils(const StencilArgs* a, int n, cudaStream_t s) {
 
 cudaError_t launch_stencil(const StencilArgs& a, cudaStream_t s) {
     if (launch_resident(&a, 1, s)) return cudaSuccess;
-    // per_pass: 0 (default) = one launch per Jacobi sweep, red-black solves
-    // in the colour-split layout where the rows allow (one launch per
-    // colour); 1 = one launch per sweep or per colour on the interleaved
+    // per_pass: 0 (default) = the whole solve resident in a cluster where the
+    // grid fits one (sf_resident.cu), else one launch per Jacobi sweep,
+    // red-black solves in the colour-split layout where the rows allow (one
+    // launch per colour); 1 = one launch per sweep or per colour on the interleaved
     // field; >= 2 = several sweeps per HBM pass: z-wavefront passes where the
     // rows suit them, else (red-black) the TMA pass. On B200 one launch per
     // sweep is the faster form: consecutive single sweeps in alternating z

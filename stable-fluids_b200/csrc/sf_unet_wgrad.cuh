@@ -25,7 +25,10 @@
 // nine taps. What it replaces (one tap a CTA, tcgen05 with M = 128, each
 // activation read 27 times from L2) ran at 7 TFLOP/s.
 //
-// What bounds it: shared memory reads (10 ldmatrix.x4 for 18 MMAs).
+// What bounds it: shared memory reads (10 ldmatrix.x4 for 18 MMAs; the tensor
+// pipe is busy half the time in a 64-channel layer at 32^3, 33 us). The bias is
+// summed from the dout fragments on the FP32 units, to nearest: as MMAs with
+// ones a 64-channel sum over 64 x 32 x 64 voxels was short by 5.2e-6, now 2.6e-7.
 //
 // The layers of 16 output channels (the full grid) take k_conv3d_wgrad_chain
 // instead. The tensor cores add their products to an FP32 accumulator rounded
@@ -36,11 +39,13 @@
 // most). The chain kernel keeps the order of the sums: K runs over the voxels
 // in memory order in blocks of 16, in as many segments as before (one wave of
 // one CTA a tap: five), and mma.sync accumulates with the bits of tcgen05.mma.
-// That leaves chains of 26,215 dependent MMAs at 128^3 as the bound (70 cycles
-// a block of 16 voxels, 20 of them the MMA's latency). The work is split by
-// taps (a CTA owns the three dx taps of one (dz, dy), 16 input channels and
-// one segment), and the layers, which do not depend on each other, share one
-// launch: 0.93 ms a layer one after the other, 1.8 ms for all five together.
+// The work is split by taps (a CTA owns the three dx taps of one (dz, dy), 16
+// input channels and one segment), and the layers, which do not depend on each
+// other, share one launch: 0.93 ms a layer one after the other, 1.8 ms for all
+// five together. What bounds it is filling shared memory: each of the nine CTAs
+// of a group brings its whole dout and in again, 8.5 GB from L2 at 128^3, 4.7
+// TB/s. The chains of 26,215 dependent MMAs leave room (70 cycles a block of 16
+// voxels, 20 of them the MMA's latency; the tensor pipe is busy 0.32 of the time).
 //
 // The whole gradient of a 128^3 pair: 26.0 -> 4.0 ms (2.8 with short chains
 // everywhere, which changes the sums).

@@ -34,11 +34,10 @@
 // updated a half-sweep at 64^3 took 2.6 us). A cell's ghost lives in
 // the other colour's array, the one its update reads.
 //
-// Waits are bounded. A CTA whose wait gives up sets the error word, tells the
-// cluster and stops; the others stop at their next wait, or finish. Whether one
-// did is known to all of them after the last cluster barrier, and then none
-// writes its block of the result. The look at the flag in every half-sweep
-// costs 0.5 to 1 % of a small grid's step (64.4 against 63.5 us at 32^3).
+// Waits are bounded. A thread whose wait gives up sets the error word, tells the
+// cluster, and sends and waits no more; the others give up at their next wait.
+// Whether one did is known to all of them after the last cluster barrier, and
+// then none writes its block of the result.
 //
 // Values, order of the sums, division and rounding are those of k_rb_half and
 // k_jacobi_vec4 (BF16 storage: rounded to BF16 at every update), so the result
@@ -102,11 +101,13 @@ __device__ __forceinline__ void store_cluster(uint32_t addr, float4 v, uint32_t 
 // Sets a word of a CTA of the cluster.
 __device__ __forceinline__ void set_remote(uint32_t addr, uint32_t rank, int v) { asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(remote(addr, rank)), "r"(v) : "memory"); }
 // tb::mbar_wait that also gives up once *stop is set (by any CTA of the cluster).
-__device__ __forceinline__ bool wait_neighbours(uint64_t* bar, unsigned parity, const volatile int* stop) {
+__device__ __forceinline__ bool wait_neighbours(uint64_t* bar, unsigned parity, unsigned polls, const volatile int* stop) {
     const unsigned addr = tb::smem_addr(bar);
-    for (unsigned it = 0; it < (1u << 26); ++it) {
+    if (tb::mbar_try_wait(addr, parity)) [[likely]] return true;
+#pragma unroll 1
+    for (unsigned it = 1; it < polls; ++it) {
         if (tb::mbar_try_wait(addr, parity)) return true;
-        if ((it & 1023u) == 1023u && *stop != 0) return false;
+        if ((it & 1023u) == 0 && *stop != 0) return false;
     }
     return false;
 }
@@ -124,8 +125,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     // two mbarriers, for the half-sweeps in turn: a neighbour may be one ahead
     uint64_t* const bar = reinterpret_cast<uint64_t*>(shared);
     float* const smem = shared + 4;
-    // two words of the pad before the first array, zero with it: a CTA of the
-    // cluster has given up; this one has (set and read between barriers only)
+    // a word of the pad before the first array, zero with it: a CTA of the
+    // cluster has given up a wait
     volatile int* const stop = reinterpret_cast<volatile int*>(smem);
     const int cs = a.py * a.pz;
     const int solve = static_cast<int>(blockIdx.x) / cs, rank = static_cast<int>(blockIdx.x) % cs;
@@ -213,19 +214,27 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
             if (count > 2) u[2] = o.z;
         }
     };
+    // A thread whose wait gives up writes no pads, arrives and waits no more (so
+    // nothing is added to barriers that stay incomplete) and goes through the
+    // remaining half-sweeps: the barriers of the CTA stay whole. The hot path has
+    // no test for it, only other loop bounds (a flag looked at in every half-sweep
+    // cost 1 to 2.5 % of a small grid's step).
+    int pad_edge = first, pad_row = tid;
+    unsigned polls = 1u << 26;
+    bool arrives = tid == 0;
     // Writes the pads that depend on the new values of colour c, at offset
     // `at`; `other` is the other colour's array of the same generation, `turn`
     // the mbarrier of the half-sweep.
     const auto write_pads = [&](int c, int at, int other, int turn) {
 #pragma unroll 1
-        for (int e = first; e < edges; e += step) {
+        for (int e = pad_edge; e < edges; e += step) {
             const int4 q = edge_at[e];
             const float4 o = *reinterpret_cast<const float4*>(field + at + q.x + k0);
             if (q.w != 0) store_cluster(static_cast<uint32_t>(q.y) + 4u * static_cast<uint32_t>(at + k0), o, static_cast<uint32_t>(q.w + turn));
             else *reinterpret_cast<float4*>(field + other + q.y + k0) = ghost_of(g, q.z, o);
         }
 #pragma unroll 1
-        for (int r = tid; r < rows; r += nt) {
+        for (int r = pad_row; r < rows; r += nt) {
             const int row = row_at[r], s = (row ^ c) & 1;
             float* const u = field + at + (row >> 1);
             float* const v = field + other + (row >> 1);
@@ -243,12 +252,15 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
     // End of half-sweep `n` (each `colours` colours of rows): the CTA's own
     // values and its neighbours' are in place.
     const auto finish = [&](int n, int colours) {
-        if (tid == 0) tb::mbar_expect_tx(&bar[n & 1], static_cast<unsigned>(colours * incoming));
+        if (arrives) tb::mbar_expect_tx(&bar[n & 1], static_cast<unsigned>(colours * incoming));
         __syncthreads();
-        if (!wait_neighbours(&bar[n & 1], static_cast<unsigned>((n >> 1) & 1), stop)) {
+        if (!wait_neighbours(&bar[n & 1], static_cast<unsigned>((n >> 1) & 1), polls, stop) && polls != 0) {
             if (a.error != nullptr) atomicOr(a.error, 1u);
-            stop[1] = 1;
             for (int r = 0; r < cs; ++r) set_remote(static_cast<uint32_t>(__cvta_generic_to_shared(smem)), static_cast<uint32_t>(r), 1);
+            pad_edge = edges;
+            pad_row = rows;
+            polls = 0;
+            arrives = false;
         }
     };
 
@@ -321,10 +333,8 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
 #pragma unroll 1
             for (int c = 0; c < 2; ++c) half(c, now + (1 - c) * array, next + c * array);
             __syncthreads();
-            const int failed = stop[1];
 #pragma unroll 1
             for (int c = 0; c < 2; ++c) write_pads(c, next + c * array, next + (1 - c) * array, 8 * (n & 1));
-            if (failed != 0) break;  // the wait before gave up; the same for every thread
             finish(n, 2);
             now = next;
         }
@@ -334,9 +344,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) k_resident(const __grid_c
             const int c = (n & 1) ^ 1;
             half(c, (1 - c) * array, c * array);
             __syncthreads();
-            const int failed = stop[1];
             write_pads(c, c * array, (1 - c) * array, 8 * (n & 1));
-            if (failed != 0) break;
             finish(n, 1);
         }
     }

@@ -1003,7 +1003,7 @@ StableFluidsResult stable_fluids_b200_attach_network(void* context, void* networ
     auto* n = static_cast<sfb::net::Net*>(network);
     if (cudaStreamSynchronize(c.stream) != cudaSuccess) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
     // the network's buffers for this grid are allocated before the capture
-    if (n != nullptr && sfb::net::prepare(n, c.coarse_b != nullptr ? c.coarse_dims() : c.dims, &c) != cudaSuccess) {
+    if (n != nullptr && sfb::net::prepare(n, c.coarse_b != nullptr ? c.coarse_dims() : c.dims, c.stream, &c) != cudaSuccess) {
         cudaGetLastError();
         return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
     }

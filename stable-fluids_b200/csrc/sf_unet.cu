@@ -318,7 +318,8 @@ Net* create_net(uint32_t seed) {
 // (325 bytes a voxel for a prediction, 700 with the gradients).
 constexpr size_t kMaxVoxels = (1ull << 31) - 4096;
 
-cudaError_t ensure_buffers(Net* n, Dims d, const void* owner = nullptr) {
+// The buffers of (d, owner), made and cleared on stream s at the first call.
+cudaError_t ensure_buffers(Net* n, Dims d, cudaStream_t s, const void* owner = nullptr) {
     if (d.nx % 4 || d.ny % 4 || d.nz % 4 || d.nx < 4 || d.ny < 4 || d.nz < 4) return cudaErrorInvalidValue;
     if (static_cast<size_t>(d.nx) * d.ny >= kMaxVoxels || static_cast<size_t>(d.nx) * d.ny * d.nz >= kMaxVoxels) return cudaErrorMemoryAllocation;
     for (auto& set : n->sets)
@@ -390,7 +391,7 @@ cudaError_t ensure_buffers(Net* n, Dims d, const void* owner = nullptr) {
         *it.p = p;
         p += (it.bytes + 255) & ~static_cast<size_t>(255);
     }
-    if (cudaMemset(b->mem, 0, total) != cudaSuccess) return cudaErrorMemoryAllocation;
+    if (cudaMemsetAsync(b->mem, 0, total, s) != cudaSuccess) return cudaErrorMemoryAllocation;
     n->buf = b.get();
     n->sets.push_back(std::move(b));
     return cudaSuccess;
@@ -520,7 +521,7 @@ cudaError_t loss_and_gradients(Net* n, const float* b, float b_factor, const flo
 
 }  // namespace
 
-cudaError_t prepare(Net* n, Dims d, const void* owner) { return ensure_buffers(n, d, owner); }
+cudaError_t prepare(Net* n, Dims d, cudaStream_t s, const void* owner) { return ensure_buffers(n, d, s, owner); }
 
 // Networks created and not yet destroyed: a context destroyed after the
 // network it was attached to must not touch it.
@@ -548,7 +549,7 @@ void release(Net* n, const void* owner) {
 }
 
 cudaError_t predict(Net* n, const float* b, float b_factor, const float* p_prev, float* p0, Dims d, cudaStream_t s, int* launches, const void* owner, unsigned* error) {
-    cudaError_t e = ensure_buffers(n, d, owner);
+    cudaError_t e = ensure_buffers(n, d, s, owner);
     if (e != cudaSuccess) return e;
     if ((e = forward(n, b, b_factor, p_prev, error != nullptr ? error : n->buf->error(), s)) != cudaSuccess) return e;
     k_unpack_output<<<blocks_for(n->buf->n0), 256, 0, s>>>(n->buf->out, p_prev, n->buf->scale, p0, n->buf->n0);
@@ -629,7 +630,7 @@ StableFluidsResult stable_fluids_b200_network_gradients(void* network, const flo
     auto* n = static_cast<Net*>(network);
     const sfb::Dims d{nx, ny, nz, 0};
     const auto s = static_cast<cudaStream_t>(stream);
-    cudaError_t e = sfb::net::ensure_buffers(n, d);
+    cudaError_t e = sfb::net::ensure_buffers(n, d, s);
     if (e == cudaSuccess) e = sfb::net::loss_and_gradients(n, divergence, cell_size * cell_size, previous_pressure, target_pressure, out_loss, s);
     if (e == cudaSuccess && out_host_gradients) e = cudaMemcpy(out_host_gradients, n->g, n->nparams * sizeof(float), cudaMemcpyDeviceToHost);
     return status(e);
@@ -640,7 +641,7 @@ StableFluidsResult stable_fluids_b200_network_train_step(void* network, const fl
     auto* n = static_cast<Net*>(network);
     const sfb::Dims d{nx, ny, nz, 0};
     const auto s = static_cast<cudaStream_t>(stream);
-    cudaError_t e = sfb::net::ensure_buffers(n, d);
+    cudaError_t e = sfb::net::ensure_buffers(n, d, s);
     if (e == cudaSuccess) e = sfb::net::loss_and_gradients(n, divergence, cell_size * cell_size, previous_pressure, target_pressure, out_loss, s);
     if (e == cudaSuccess) e = sfb::net::adam_step(n, learning_rate, s);
     return status(e);

@@ -18,12 +18,13 @@ constexpr int kPredictKernels = 19;
 // refreshes the BF16 copies; resets the optimizer state.
 cudaError_t set_parameters(Net* n, const float* host);
 
-// Allocates the activation buffers for grid d and `owner` (synchronous; call
-// it before a stream capture that will contain predict()). Each owner (an
+// Allocates the activation buffers for grid d and `owner` and clears them on
+// stream s, the one that predict() will run on (call it before a stream
+// capture that will contain predict()). Each owner (an
 // attached context) gets inference-only buffers of its own, so that contexts
 // sharing the network can predict concurrently; owner null is the network's
 // own set. Grid sides must be multiples of 4.
-cudaError_t prepare(Net* n, Dims d, const void* owner);
+cudaError_t prepare(Net* n, Dims d, cudaStream_t s, const void* owner);
 
 // Frees the buffer sets of `owner` (its step graphs must be gone or rebuilt).
 void release(Net* n, const void* owner);

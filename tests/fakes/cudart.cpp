@@ -42,6 +42,10 @@ std::map<void*, size_t> blocks;
 std::map<std::string, int> executed;  // kernels that ran outside a graph, by name
 int executed_total = 0, refused = 0, occupancy_queries = 0;
 bool take_clusters = true;
+// work on the default stream that nothing has waited for, and launches on
+// non-blocking streams (all that the library makes) beside it
+bool default_stream_busy = false;
+int unordered = 0;
 size_t patch_size = 0, patch_offset = 0;
 unsigned patch_value = 0;
 Stream null_stream;
@@ -65,6 +69,8 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t shared, cudaStre
         ++refused;
         return keep(cudaErrorInvalidValue);
     }
+    if (s != nullptr && default_stream_busy) ++unordered;
+    if (s == nullptr) default_stream_busy = true;
     if (Graph* g = of(s)->capture) {
         ++g->kernels;
     } else {
@@ -89,6 +95,7 @@ extern "C" {
 void fake_set_device(int d) { current = d; }
 int fake_refused() { return refused; }
 int fake_occupancy_queries() { return occupancy_queries; }
+int fake_unordered() { return unordered; }
 int fake_executed() { return executed_total; }
 int fake_executed_of(const char* part) {
     int n = 0;
@@ -143,7 +150,10 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) {
     std::strcpy(p->name, "fake");
     return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() {
+    default_stream_busy = false;
+    return cudaSuccess;
+}
 cudaError_t cudaGetLastError() {
     const cudaError_t e = last;
     last = cudaSuccess;
@@ -211,10 +221,11 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
 }
 // fresh memory is zero already: clearing the large blocks would only touch them
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t s) {
+    if (s == nullptr) default_stream_busy = true;
     if (of(s)->capture == nullptr && n <= (1u << 20)) std::memset(d, v, n);
     return cudaSuccess;
 }
-cudaError_t cudaMemset(void* d, int v, size_t n) { return cudaMemsetAsync(d, v, n, nullptr); }
+cudaError_t cudaMemset(void* d, int v, size_t n) { return cudaMemsetAsync(d, v, n, nullptr); }  // returns before it has run
 
 // ---- streams, events, graphs ----
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
@@ -225,7 +236,10 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
     delete of(s);
     return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    if (s == nullptr) default_stream_busy = false;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t s, cudaStreamCaptureMode) {
     of(s)->capture = new Graph;

@@ -262,7 +262,9 @@ cudaError_t wgrad_any(int cin, int cout, const __nv_bfloat16* in, const __nv_bfl
 
 // Copies FP32 master parameters from the host and refreshes the BF16 copies.
 cudaError_t set_parameters(Net* n, const float* host) {
-    cudaError_t e = cudaMemcpy(n->w, host, n->nparams * sizeof(float), cudaMemcpyHostToDevice);
+    // a training step returns while its optimizer still runs on its stream
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(n->w, host, n->nparams * sizeof(float), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return e;
     n->adam_t = 0;
     // An Adam pass with lr = 0 and zero gradients leaves w unchanged and
@@ -610,8 +612,10 @@ StableFluidsResult stable_fluids_b200_network_parameters(void* network, uint64_t
     if (network == nullptr) return STABLE_FLUIDS_RESULT_BACKEND_FAILURE;
     auto* n = static_cast<Net*>(network);
     if (out_count) *out_count = n->nparams;
-    if (out_host_values) return status(cudaMemcpy(out_host_values, n->w, n->nparams * sizeof(float), cudaMemcpyDeviceToHost));
-    return STABLE_FLUIDS_RESULT_OK;
+    if (out_host_values == nullptr) return STABLE_FLUIDS_RESULT_OK;
+    cudaError_t e = cudaDeviceSynchronize();  // the optimizer of a training step on its stream
+    if (e == cudaSuccess) e = cudaMemcpy(out_host_values, n->w, n->nparams * sizeof(float), cudaMemcpyDeviceToHost);
+    return status(e);
 }
 
 StableFluidsResult stable_fluids_b200_network_set_parameters(void* network, const float* host_values) {

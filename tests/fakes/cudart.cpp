@@ -42,9 +42,11 @@ std::map<void*, size_t> blocks;
 std::map<std::string, int> executed;  // kernels that ran outside a graph, by name
 int executed_total = 0, refused = 0, occupancy_queries = 0;
 bool take_clusters = true;
-// work on the default stream that nothing has waited for, and launches on
-// non-blocking streams (all that the library makes) beside it
+// work that nothing has waited for, on the default stream and on non-blocking
+// ones (all that the library makes), and what was done beside it: launches on a
+// non-blocking stream, copies and launches on the default one
 bool default_stream_busy = false;
+std::set<cudaStream_t> busy;
 int unordered = 0;
 size_t patch_size = 0, patch_offset = 0;
 unsigned patch_value = 0;
@@ -70,12 +72,16 @@ cudaError_t launch(const void* f, dim3 grid, dim3 block, size_t shared, cudaStre
         return keep(cudaErrorInvalidValue);
     }
     if (s != nullptr && default_stream_busy) ++unordered;
-    if (s == nullptr) default_stream_busy = true;
+    if (s == nullptr) {
+        if (!busy.empty()) ++unordered;
+        default_stream_busy = true;
+    }
     if (Graph* g = of(s)->capture) {
         ++g->kernels;
     } else {
         ++executed_total;
         ++executed[names[f]];
+        if (s != nullptr) busy.insert(s);
     }
     return cudaSuccess;
 }
@@ -152,6 +158,7 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) {
 }
 cudaError_t cudaDeviceSynchronize() {
     default_stream_busy = false;
+    busy.clear();
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {
@@ -216,6 +223,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    if (!busy.empty()) ++unordered;
     copy(d, s, n);
     return cudaSuccess;
 }
@@ -238,6 +246,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     if (s == nullptr) default_stream_busy = false;
+    busy.erase(s);
     return cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }

@@ -1,7 +1,8 @@
-"""The network's buffers are cleared before the first pass on them starts,
-whichever stream it runs on: nothing is launched on a stream of the caller's
-while work on the default stream is under way (a CUDA runtime without a GPU,
-fake_cuda.py, keeps the account)."""
+"""What the network does on the default stream is in order with the passes on
+the caller's streams, which do not wait for it: its buffers are cleared before
+the first pass on them, and parameters are read and set when no step of the
+optimizer is under way (a CUDA runtime without a GPU, fake_cuda.py, keeps the
+account)."""
 
 import ctypes
 
@@ -34,4 +35,20 @@ def test_first_step_of_a_learned_context(sf, tmp_path):
     assert lib.stable_fluids_step_cuda(ctx) == sf.RESULT_OK
     assert lib.fake_unordered() == 0
     lib.stable_fluids_destroy_context_cuda(ctx)
+    lib.stable_fluids_b200_network_destroy(net)
+
+
+def test_parameters_after_a_training_step(sf, tmp_path):
+    lib = fake_cuda.load(sf, tmp_path)
+    stream, net, count = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_uint64()
+    assert lib.cudaStreamCreateWithFlags(ctypes.byref(stream), 1) == 0
+    assert lib.stable_fluids_b200_network_create(1, ctypes.byref(net)) == sf.RESULT_OK
+    lib.stable_fluids_b200_network_parameters(net, ctypes.byref(count), None)
+    values = (ctypes.c_float * count.value)()
+    n = (16, 12, 8)
+    field = (ctypes.c_float * (n[0] * n[1] * n[2]))()
+    for use in (lib.stable_fluids_b200_network_set_parameters, lambda h, v: lib.stable_fluids_b200_network_parameters(h, None, v)):
+        assert lib.stable_fluids_b200_network_train_step(net, field, field, field, *n, 1.0, 1e-3, None, stream) == sf.RESULT_OK
+        assert use(net, values) == sf.RESULT_OK
+        assert lib.fake_unordered() == 0
     lib.stable_fluids_b200_network_destroy(net)

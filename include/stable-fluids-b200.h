@@ -179,7 +179,9 @@ STABLE_FLUIDS_API StableFluidsResult stable_fluids_b200_get_step_info(void* cont
  * and output channels 1..15 of the last are padding (zero, never updated).
  *
  * A network object serves one stream at a time (its activation buffers are
- * shared by every call); all entry points except predict are synchronous.
+ * shared by every call); all entry points except predict are synchronous, but
+ * for train_step's update of the parameters, which runs on in that stream (the
+ * entry points that read or set them wait for it).
  * When a kernel gives up one of its bounded waits, gradients and train_step
  * return BACKEND_FAILURE and leave the parameters as they were (after predict
  * on a grid: the next of them on that grid; in a step:

@@ -90,6 +90,7 @@ class Simulation:
         torch = self._torch
         if isinstance(values, torch.Tensor):
             t = values
+            self.stream.wait_stream(torch.cuda.current_stream(self.device))  # which has computed it
             if t.device != self.device or t.dtype != torch.float32 or not t.is_contiguous():
                 with torch.cuda.stream(self.stream):
                     t = t.to(self.device, torch.float32).contiguous()
